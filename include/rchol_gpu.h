@@ -132,12 +132,13 @@ int rchol_gpu_factor_export(rchol_factor_t G, int64_t *row_ptr, int64_t *col_idx
 /* Pivots d of the factorization (length n), G = L sqrt(D). */
 int rchol_gpu_factor_pivots(rchol_factor_t G, double *d);
 /* Shape of the triangular-solve plan of the forward (transpose = 0) or
- * backward solve: stages (kernel pairs in sequence), pieces, and the
- * sequential 32-row block steps on the critical path.  No counterpart in
+ * backward solve: stages (kernels in sequence), pieces, and the sequential
+ * block steps on the critical path (32 to 512 rows each).  No counterpart in
  * the reference. */
 int rchol_gpu_factor_plan_info(rchol_factor_t G, int transpose, int64_t *stages, int64_t *pieces, int64_t *steps);
-/* Autotuning of the solves on this factor: times the preconditioner with
- * alternative launch choices (L2 prefetch distance and ring depth of the
+/* Autotuning of the preconditioner that PCG applies with this factor (with G
+ * in FP64 there are no launch choices: it is timed and nothing changes):
+ * times the preconditioner with alternative launch choices (L2 prefetch distance and ring depth of the
  * pipeline format, warps per thread block and prefetch of the warp format)
  * and keeps the fastest for all later solves with G.  ms_before / ms_after:
  * preconditioner time with the choices on entry / chosen; knobs (4 ints, may

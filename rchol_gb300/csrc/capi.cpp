@@ -43,6 +43,7 @@ void check_solve_status(cudaStream_t s);
 void wait_selftest(uint32_t polls, cudaStream_t s);
 void edge_grad(int64_t m, const int64_t *ei, const int64_t *ej, const double *lam, const double *x, double *g,
                cudaStream_t s);
+std::pair<double, double> tune_plan(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
 void precond_noalloc(const rchol_factor_s &F, const double *r, double *z, cudaStream_t s);
 
 }  // namespace rchol
@@ -264,6 +265,13 @@ int64_t rchol_gpu_factor_nnz(rchol_factor_t G) { return G ? G->nnz : -1; }
 int rchol_gpu_factor_plan_info(rchol_factor_t G, int transpose, int64_t *stages, int64_t *pieces, int64_t *steps) {
   API_BEGIN
   RCHOL_CHECK_ARG(G && G->plan, "null factor");
+  if (G->plan->blocked) {
+    const BlkDir &B = transpose ? G->plan->bbwd : G->plan->bfwd;
+    if (stages) *stages = (int64_t)B.stages.size();
+    if (pieces) *pieces = B.npieces;
+    if (steps) *steps = B.steps;
+    return RCHOL_OK;
+  }
   const StreamDir &D = transpose ? G->plan->sbwd : G->plan->sfwd;
   if (stages) *stages = (int64_t)D.stage_ptr.size() - 1;
   if (pieces) *pieces = D.stage_ptr.empty() ? 0 : D.stage_ptr.back();
@@ -275,7 +283,7 @@ int rchol_gpu_factor_tune(rchol_factor_t G, double *ms_before, double *ms_after,
   API_BEGIN
   RCHOL_CHECK_ARG(G && G->plan, "null factor");
   std::lock_guard<std::mutex> guard(G->plan->lock);
-  const std::pair<double, double> t = tune_solves(*G, *G->plan, 0);
+  const std::pair<double, double> t = tune_plan(*G, *G->plan, 0);
   if (ms_before) *ms_before = t.first;
   if (ms_after) *ms_after = t.second;
   if (knobs) {

@@ -63,6 +63,70 @@ struct StreamDir {
   int64_t steps = 0;                 // sequential block steps on the critical path
 };
 
+// ---- block plan (blocks.cu) -------------------------------------------------------
+//
+// One direction of the triangular solves as sequential steps of up to 512
+// rows, each step one exact triangular inverse.  A piece (a tree node, cut at
+// kBlkMaxRows rows) is solved by a cluster of C thread blocks.  Positions
+// count a piece's rows in processing order (backward: from its last row);
+// block s holds positions [s B, (s+1) B), and its rows go to the ranks of the
+// cluster in groups of four (group q to rank q mod C).  The entries in
+// earlier blocks are in record rec0 + s C + rank, the inverse's rows at
+// inv0 + (blk0 + s) C + rank times the stage's stride.
+
+constexpr int kBlkMaxRows = 16384;  // a piece's unknowns in shared memory: 64 KB in FP32, 128 KB in FP64
+constexpr int kBlkMaxGroups = 64;   // 4-row groups of a thread block
+
+struct BlkPiece {
+  int64_t begin;   // first row
+  int32_t rows;
+  int32_t nblocks;
+  int64_t rec0;    // first record
+  int64_t blk0;    // blocks of the stage before it
+};
+
+struct BlkStage {
+  int piece0 = 0, npieces = 0;
+  int C = 1, B = 32;
+  int gl = 32;            // lanes of a 4-row group (row threads; a quarter of them per row)
+  int helpers = 0;        // threads that prepare the next block (clusters)
+  int nv = 1;             // vectors of the inverse per thread and row
+  int maxrows = 0;        // longest piece
+  int64_t rows = 0;       // rows of all pieces
+  int64_t erow0 = 0;      // their place in erow
+  bool fused = false;     // its records hold external entries
+  int late_lanes = 0;     // > 0: its late external entries are summed before it
+  int slot = 0;           // bytes of a ring slot
+  int ring = 4;
+  size_t smem = 0;
+  int64_t inv0 = 0;       // its inverses (values)
+  int64_t stride = 0;     // values per (block, rank)
+  int32_t goff[kBlkMaxGroups + 1] = {};  // first vector of a group
+};
+
+struct BlkExt {  // CSR over the matrix's rows
+  DevBuf<int64_t> rp;
+  DevBuf<int32_t> ci;
+  DevBuf<double> v64;
+  DevBuf<float> v32;
+  int lanes = 8;  // per row
+};
+
+struct BlkDir {
+  std::vector<BlkStage> stages;
+  DevBuf<BlkPiece> pieces;
+  DevBuf<int64_t> rec_off;
+  DevBuf<unsigned char> recs;
+  DevBuf<double> inv64;
+  DevBuf<float> inv32;
+  // external entries summed by kernels of their own: those in columns of the
+  // first stage after it, for all later rows; the rest before a stage
+  BlkExt early, late;
+  DevBuf<int32_t> erow;  // the later stages' rows
+  int64_t early_rows = 0;
+  int64_t steps = 0, npieces = 0;
+};
+
 // Workspace and captured CUDA graph of one PCG iteration for a given matrix
 // and number of right-hand sides (solve.cu).
 struct PcgWork {
@@ -122,6 +186,9 @@ struct SolvePlan {
   double tuned_ms = 0.0;  // preconditioner time with the tuned knobs (0: not tuned)
   std::vector<std::unique_ptr<PcgWork>> pcg;
   std::vector<std::unique_ptr<SegWork>> seg;
+  unsigned int *status = nullptr;  // status word of the solve kernels
+  bool blocked = false;    // the solves run on bfwd / bbwd (else, and in an FP32 PCG, on the record streams)
+  BlkDir bfwd, bbwd;
   StreamDir sfwd, sbwd;
   StreamDir kfwd, kbwd;    // pieces for up to 32 right-hand sides (built on first use)
   bool kbuilt = false;
@@ -134,14 +201,23 @@ struct SolvePlan {
   DevBuf<float> acck32;
 };
 
+// Block plan of both directions; false if G's rows are too dense for it.
+bool build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
+// Solve with G (upper = false) or G^T for one right-hand side; acc: n values
+// of G's precision.
+void block_trsv(const rchol_factor_s &F, const SolvePlan &P, bool upper, const double *in64, const float *in32,
+                double *out64, float *out32, void *acc, cudaStream_t s);
+// Device address of the status word of the solve kernels (current device).
+unsigned int *solve_status_word();
 void build_streams(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
 void build_streams_k(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
 // Solve with G (upper = false) or G^T for k right-hand sides, n x k
 // row-major, in groups of up to 32 columns.
 void stream_trsv_k(const rchol_factor_s &F, const SolvePlan &P, bool upper, const double *in64,
                    const float *in32, double *out64, float *out32, int k, cudaStream_t s);
+// acc: n values of G's precision.
 void stream_trsv(const rchol_factor_s &F, const SolvePlan &P, bool upper, const double *in64,
-                 const float *in32, double *out64, float *out32, cudaStream_t s);
+                 const float *in32, double *out64, float *out32, void *acc, cudaStream_t s);
 // Times the preconditioner under alternative SolveKnobs and keeps the
 // fastest; returns {ms with the knobs on entry, ms with the chosen ones}.
 std::pair<double, double> tune_solves(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);

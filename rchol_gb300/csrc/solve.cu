@@ -10,6 +10,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <numeric>
 #include <vector>
 
@@ -400,7 +401,28 @@ void finish_factor(rchol_factor_s &F, cudaStream_t s) {
 void build_plan(rchol_factor_s &F, cudaStream_t s) {
   auto P = new SolvePlan();
   try {
-    build_streams(F, *P, s);
+    P->status = solve_status_word();
+    // The solves run in large blocks (blocks.cu) where G allows it and
+    // RCHOL_TRSV_FORMAT does not ask for one of trsv.cu's record formats.  A
+    // PCG with G in FP32 stays with the record streams: its iterates follow
+    // the FP32 rounding of the preconditioner (of 40 systems solved to 1e-8
+    // five took an iteration more or less with another order of the sums), so
+    // a solve gives the same iterates as ever.  Both plans are then built at
+    // once, the records by the host's threads and the blocks by the GPU.
+    const bool blocks = !getenv("RCHOL_TRSV_FORMAT"), fp32 = F.precision == RCHOL_PREC_FP32;
+    std::future<bool> other;
+    if (blocks && fp32) {
+      int dev = 0;
+      RCHOL_CUDA(cudaGetDevice(&dev));
+      other = std::async(std::launch::async, [&F, P, s, dev] {
+        RCHOL_CUDA(cudaSetDevice(dev));
+        return build_blocks(F, *P, s);
+      });
+    } else {
+      P->blocked = blocks && build_blocks(F, *P, s);
+    }
+    if (fp32 || !P->blocked) build_streams(F, *P, s);
+    if (other.valid()) P->blocked = other.get();
   } catch (...) {
     delete P;
     throw;
@@ -425,15 +447,41 @@ static void ensure_scratch(SolvePlan &P, bool fp32, int64_t count) {
   }
 }
 
+// One right-hand side, in large blocks or by the record streams.  acc: n
+// values of G's precision.
+static void trsv_one(const rchol_factor_s &F, const SolvePlan &P, bool blocks, bool upper, const double *in64,
+                     const float *in32, double *out64, float *out32, void *acc, cudaStream_t s) {
+  if (blocks) block_trsv(F, P, upper, in64, in32, out64, out32, acc, s);
+  else stream_trsv(F, P, upper, in64, in32, out64, out32, acc, s);
+}
+
+// z = (G G^T)^-1 r with the intermediate vector in y64 or y32.
+static void precond_one(const rchol_factor_s &F, const SolvePlan &P, bool blocks, const double *r, double *z,
+                        double *y64, float *y32, void *acc, cudaStream_t s) {
+  trsv_one(F, P, blocks, false, r, nullptr, y64, y32, acc, s);
+  trsv_one(F, P, blocks, true, y64, y32, z, nullptr, acc, s);
+}
+
+// The plan's partial-sum vector, sized for n values.
+static void *ensure_acc(SolvePlan &P, bool fp32, int64_t n) {
+  if (fp32) {
+    if (P.acc32.n < (size_t)n) P.acc32.alloc(n);
+    return P.acc32.p;
+  }
+  if (P.acc64.n < (size_t)n) P.acc64.alloc(n);
+  return P.acc64.p;
+}
+
 // The preconditioner with the plan's buffers already sized (inside PCG).
-static void precond_ready(const rchol_factor_s &F, const double *r, double *z, int k, cudaStream_t s);
+static void precond_ready(const rchol_factor_s &F, bool blocks, const double *r, double *z, int k, cudaStream_t s);
 
 void trsv(const rchol_factor_s &F, bool upper, const double *in, double *out, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
-  ensure_scratch(P, F.precision == RCHOL_PREC_FP32, F.n * k);
+  const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  ensure_scratch(P, fp32, F.n * k);
   if (k == 1) {
-    stream_trsv(F, P, upper, in, nullptr, out, nullptr, s);
+    trsv_one(F, P, P.blocked, upper, in, nullptr, out, nullptr, ensure_acc(P, fp32, F.n), s);
     return;
   }
   build_streams_k(F, P, s);
@@ -445,20 +493,17 @@ void precond(const rchol_factor_s &F, const double *r, double *z, int k, cudaStr
   std::lock_guard<std::mutex> guard(P.lock);
   ensure_scratch(P, F.precision == RCHOL_PREC_FP32, F.n * k);
   if (k > 1) build_streams_k(F, P, s);
-  precond_ready(F, r, z, k, s);
+  precond_ready(F, P.blocked, r, z, k, s);
 }
 
-static void precond_ready(const rchol_factor_s &F, const double *r, double *z, int k, cudaStream_t s) {
+// The preconditioner of the PCG loops (see build_plan).
+static bool pcg_blocks(const rchol_factor_s &F) { return F.plan->blocked && F.precision != RCHOL_PREC_FP32; }
+
+static void precond_ready(const rchol_factor_s &F, bool blocks, const double *r, double *z, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   if (k == 1) {
-    if (fp32) {
-      stream_trsv(F, P, false, r, nullptr, nullptr, P.ytmp32.p, s);
-      stream_trsv(F, P, true, nullptr, P.ytmp32.p, z, nullptr, s);
-    } else {
-      stream_trsv(F, P, false, r, nullptr, P.ytmp.p, nullptr, s);
-      stream_trsv(F, P, true, P.ytmp.p, nullptr, z, nullptr, s);
-    }
+    precond_one(F, P, blocks, r, z, P.ytmp.p, P.ytmp32.p, ensure_acc(P, fp32, F.n), s);
     return;
   }
   if (fp32) {
@@ -468,6 +513,98 @@ static void precond_ready(const rchol_factor_s &F, const double *r, double *z, i
     stream_trsv_k(F, P, false, r, nullptr, P.ytmp.p, nullptr, k, s);
     stream_trsv_k(F, P, true, P.ytmp.p, nullptr, z, nullptr, k, s);
   }
+}
+
+// ---- preconditioner apply without allocation --------------------------------------------
+//
+// Some callers cannot allocate device memory at solve time: code that runs
+// under a fixed memory budget decided at start-up, allocator-free real-time
+// loops, or hosts that own all device memory themselves.  For them the
+// preconditioner z = (G G^T)^-1 r can run with its two scratch vectors (the
+// partial sums and the intermediate y = G^-1 r) in this fixed, file-scope
+// device array instead of buffers allocated with the factor's plan.  Every
+// GPU that loads the library holds the array until the process exits.
+// The array is shared by all calls and keeps the last call's contents; nothing
+// in it has to start at zero (both vectors are fully written before they are
+// read), and calls that overlap on the GPU race on it.
+constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;  // 16 MiB
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+
+namespace {
+constexpr size_t up16(size_t x) { return (x + 15) & ~size_t(15); }
+constexpr int kNoAllocDevices = 128;
+std::mutex g_noalloc_mutex;
+void *g_noalloc_ptr[kNoAllocDevices] = {};  // device address of the array, per device ordinal
+}  // namespace
+
+size_t noalloc_scratch_bytes() { return kNoAllocScratchBytes; }
+
+// Set-up on the current device: the array's host-side name is only a
+// stand-in, so its device address is looked up with the device current.  The
+// first call on a device does this (it should come before any stream
+// capture); later calls whose stream is not capturing look it up again, so a
+// device reset (which gives the array a new address) leaves no stale pointer.
+static void *noalloc_scratch_address(cudaStream_t s) {
+  int dev = 0;
+  RCHOL_CUDA(cudaGetDevice(&dev));
+  RCHOL_CHECK_ARG(dev >= 0 && dev < kNoAllocDevices, "device ordinal out of range");
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+    (void)cudaGetLastError();  // e.g. the legacy stream while another stream captures
+    cs = cudaStreamCaptureStatusActive;
+  }
+  std::lock_guard<std::mutex> guard(g_noalloc_mutex);
+  if (!g_noalloc_ptr[dev] || cs == cudaStreamCaptureStatusNone) {
+    void *p = nullptr;
+    RCHOL_CUDA(cudaGetSymbolAddress(&p, g_noalloc_scratch));
+    g_noalloc_ptr[dev] = p;
+  }
+  return g_noalloc_ptr[dev];
+}
+
+void precond_noalloc(const rchol_factor_s &F, const double *r, double *z, cudaStream_t s) {
+  const int64_t n = F.n;
+  const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  const size_t vsz = fp32 ? 4 : 8;
+  const size_t acc_bytes = up16((size_t)n * vsz);
+  if (2 * acc_bytes > kNoAllocScratchBytes)
+    throw Error(RCHOL_ERR_INVALID, "n = " + std::to_string(n) + " needs " + std::to_string(2 * acc_bytes) +
+                                       " bytes of scratch; the allocation-free entry point has " +
+                                       std::to_string(kNoAllocScratchBytes) + " (n <= " +
+                                       std::to_string(kNoAllocScratchBytes / (2 * vsz)) + " for this precision)");
+  unsigned char *base = static_cast<unsigned char *>(noalloc_scratch_address(s));
+  void *y = base + acc_bytes;
+  precond_one(F, *F.plan, F.plan->blocked, r, z, fp32 ? nullptr : static_cast<double *>(y), fp32 ? static_cast<float *>(y) : nullptr,
+              base, s);
+}
+
+// rchol_gpu_factor_tune: the launch choices of the preconditioner that PCG
+// applies.  The block plan has none: it is timed and left as it is.
+std::pair<double, double> tune_plan(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
+  if (!pcg_blocks(F)) return tune_solves(F, P, s);
+  const int64_t n = F.n;
+  const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  DevBuf<double> r(n), z(n), y64(fp32 ? 0 : n);
+  DevBuf<float> y32(fp32 ? n : 0);
+  void *acc = ensure_acc(P, fp32, n);
+  RCHOL_CUDA(cudaMemsetAsync(r.p, 0, r.bytes(), s));
+  cudaEvent_t e0, e1;
+  RCHOL_CUDA(cudaEventCreate(&e0));
+  RCHOL_CUDA(cudaEventCreate(&e1));
+  float best = 1e30f;
+  for (int rep = 0; rep < 4; ++rep) {
+    RCHOL_CUDA(cudaEventRecord(e0, s));
+    precond_one(F, P, true, r.p, z.p, y64.p, y32.p, acc, s);
+    RCHOL_CUDA(cudaEventRecord(e1, s));
+    RCHOL_CUDA(cudaEventSynchronize(e1));
+    float ms = 0.f;
+    RCHOL_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    if (rep) best = std::min(best, ms);
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  P.tuned_ms = best;
+  return {best, best};
 }
 
 void spmv_public(const rchol_matrix_s &A, const double *x, double *y, int k, cudaStream_t s) {
@@ -591,7 +728,7 @@ static void pcg_iteration(const rchol_matrix_s &A, const rchol_factor_s &F, PcgW
   const int k = w.k;
   const int64_t n = A.n, nk = n * k;
   const unsigned eb = (unsigned)((nk + 255) / 256);
-  precond_ready(F, w.r.p, w.z.p, k, s);
+  precond_ready(F, pcg_blocks(F), w.r.p, w.z.p, k, s);
   reduce_kernel<RED_DOT><<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, st, w.r.p, w.z.p, nullptr, nullptr, nullptr);
   finalize_kernel<<<k, RED_THREADS, 0, s>>>(st, FIN_BETA, 0, nullptr);
   pupdate_kernel<<<eb, 256, 0, s>>>(nk, st, w.p.p, w.z.p);
@@ -615,10 +752,7 @@ static void pcg_impl(const rchol_matrix_s &A, const rchol_factor_s &F, const dou
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   ensure_scratch(P, fp32, nk);
   if (k > 1) build_streams_k(F, P, s);
-  if (fp32 ? P.acc32.n < (size_t)n : P.acc64.n < (size_t)n) {
-    if (fp32) P.acc32.alloc(n);
-    else P.acc64.alloc(n);
-  }
+  ensure_acc(P, fp32, n);
   PcgWork &w = pcg_workspace(A, F, k);
   PcgState st = pcg_state(w);
   cudaStream_t ws = w.stream;
@@ -887,10 +1021,7 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
   const int64_t n = A.n;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   ensure_scratch(P, fp32, n);
-  if (fp32 ? P.acc32.n < (size_t)n : P.acc64.n < (size_t)n) {
-    if (fp32) P.acc32.alloc(n);
-    else P.acc64.alloc(n);
-  }
+  ensure_acc(P, fp32, n);
   SegWork &w = seg_workspace(A, F, nseg, seg);
   SegState st = seg_state(w);
   const unsigned S = (unsigned)nseg;
@@ -908,7 +1039,7 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
     cudaGraph_t g = nullptr;
     RCHOL_CUDA(cudaStreamBeginCapture(ws, cudaStreamCaptureModeThreadLocal));
     try {
-      precond_ready(F, w.r.p, w.z.p, 1, ws);
+      precond_ready(F, pcg_blocks(F), w.r.p, w.z.p, 1, ws);
       seg_beta_kernel<<<S, SEG_THREADS, 0, ws>>>(st, w.r.p, w.z.p, w.p.p);
       spmv(A, w.p.p, w.q.p, 1, ws);
       seg_alpha_kernel<<<S, SEG_THREADS, 0, ws>>>(st, w.p.p, w.q.p, w.x.p, w.r.p);

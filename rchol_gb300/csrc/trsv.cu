@@ -1,4 +1,7 @@
-// Block triangular solves with G (forward) and G^T (backward).
+// Block triangular solves with G (forward) and G^T (backward) from streams of
+// 32-row records: several right-hand sides at once, factors whose rows are too
+// dense for the large blocks of blocks.cu or whose entries have mixed signs,
+// and the formats that RCHOL_TRSV_FORMAT names.
 //
 // Replaces the two MKL trsv calls of c++/util/pcg.cpp:141-159.
 //
@@ -36,6 +39,7 @@
 #include <utility>
 #include <vector>
 
+#include "bulk.hpp"
 #include "common.hpp"
 #include "host.hpp"
 #include "plan.hpp"
@@ -935,55 +939,6 @@ void build_pipe_piece(const std::vector<int64_t> &rp, const std::vector<int32_t>
     for (int r = 0; r < BS; ++r)
       for (int c = 0; c < BS; ++c) P.sparse += (N1[r][c] != 0.0) + (N2[r][c] != 0.0);
   }
-}
-
-// ---- bulk copies into shared memory ----------------------------------------------------
-//
-// Records stream into a ring of shared-memory slots with cp.async.bulk (the
-// copy engine moves a whole record; no thread issues 16-byte pieces), one
-// mbarrier per slot counting the record's bytes.  Far-ahead records are
-// prefetched into L2.  Every wait is bounded: after kWaitLimit polls the
-// kernel records bit 0 in g_solve_status, stops issuing copies, waits
-// (bounded) for the ones in flight and finishes without using the data.
-
-constexpr uint32_t kWaitLimit = 1u << 22;
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-// orders this thread's earlier shared-memory accesses before later async-proxy (bulk copy) ones
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes)
-               : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-__device__ __forceinline__ void prefetch_l2(const void *src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Waits for the phase of `parity` to complete; false after kWaitLimit polls.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kWaitLimit; ++i)
-    if (mbar_test(bar, parity)) return true;
-  return false;
 }
 
 // Byte offsets of a piece's records, held by the 32 lanes of one warp: lane j
@@ -2065,7 +2020,7 @@ static void build_streams_width(const rchol_factor_s &F, int kwidth, StreamDir &
   RCHOL_CUDA(cudaStreamSynchronize(s));
   // Schedule knob (tuning only; every setting solves exactly the same
   // system): RCHOL_TRSV_FORMAT = 0 warp format everywhere, 1 by stage
-  // (default: warp format where a depth has many nodes, pipeline format
+  // (the choice without the variable: warp format where a depth has many nodes, pipeline format
   // at the top of the tree), 2 pipeline format everywhere.
   int fmt_mode = 1;
   if (const char *e = getenv("RCHOL_TRSV_FORMAT")) fmt_mode = std::max(0, std::min(2, atoi(e)));
@@ -2233,6 +2188,12 @@ __global__ void wait_selftest_kernel(uint32_t polls) {
 }
 }  // namespace
 
+unsigned int *solve_status_word() {
+  void *p = nullptr;
+  RCHOL_CUDA(cudaGetSymbolAddress(&p, g_solve_status));
+  return static_cast<unsigned int *>(p);
+}
+
 uint32_t take_solve_status(cudaStream_t s) {
   RCHOL_CUDA(cudaStreamSynchronize(s));
   uint32_t v = 0;
@@ -2325,19 +2286,17 @@ std::pair<double, double> tune_solves(const rchol_factor_s &F, SolvePlan &P, cud
   return {before, best};
 }
 
-void stream_trsv(const rchol_factor_s &F, const SolvePlan &P, bool upper, const double *in64,
-                 const float *in32, double *out64, float *out32, cudaStream_t s) {
-  SolvePlan &Pm = const_cast<SolvePlan &>(P);
-  const int64_t n = F.n;
+void stream_trsv(const rchol_factor_s &F, const SolvePlan &P, bool upper, const double *in64, const float *in32,
+                 double *out64, float *out32, void *acc, cudaStream_t s) {
   if (F.precision == RCHOL_PREC_FP32) {
-    if (Pm.acc32.n < (size_t)n) Pm.acc32.alloc(n);
-    if (in64 && out32) launch_streams<float, double, float>(P, upper, in64, out32, Pm.acc32.p, s);
-    else if (in32 && out64) launch_streams<float, float, double>(P, upper, in32, out64, Pm.acc32.p, s);
-    else if (in64 && out64) launch_streams<float, double, double>(P, upper, in64, out64, Pm.acc32.p, s);
+    float *a = static_cast<float *>(acc);
+    if (in64 && out32) launch_streams<float, double, float>(P, upper, in64, out32, a, s);
+    else if (in32 && out64) launch_streams<float, float, double>(P, upper, in32, out64, a, s);
+    else if (in64 && out64) launch_streams<float, double, double>(P, upper, in64, out64, a, s);
     else throw Error(RCHOL_ERR_INTERNAL, "unsupported triangular-solve operand types");
   } else {
-    if (Pm.acc64.n < (size_t)n) Pm.acc64.alloc(n);
-    if (in64 && out64) launch_streams<double, double, double>(P, upper, in64, out64, Pm.acc64.p, s);
+    double *a = static_cast<double *>(acc);
+    if (in64 && out64) launch_streams<double, double, double>(P, upper, in64, out64, a, s);
     else throw Error(RCHOL_ERR_INTERNAL, "unsupported triangular-solve operand types");
   }
 }
@@ -2399,76 +2358,6 @@ void stream_trsv_k(const rchol_factor_s &F, const SolvePlan &P, bool upper, cons
         launch_streams_k<double, double, double>(P, upper, in64 + j0, out64 + j0, P.acck64.p, kg, k, s);
       else throw Error(RCHOL_ERR_INTERNAL, "unsupported triangular-solve operand types");
     }
-  }
-}
-
-// ---- preconditioner apply without allocation --------------------------------------------
-//
-// Some callers cannot allocate device memory at solve time: code that runs
-// under a fixed memory budget decided at start-up, allocator-free real-time
-// loops, or hosts that own all device memory themselves.  For them the
-// preconditioner z = (G G^T)^-1 r can run with its two scratch vectors (the
-// partial sums and the intermediate y = G^-1 r) in this fixed, file-scope
-// device array instead of buffers allocated with the factor's plan.  Every
-// GPU that loads the library holds the array until the process exits.
-// The array is shared by all calls and keeps the last call's contents; nothing
-// in it has to start at zero (both vectors are fully written before they are
-// read), and calls that overlap on the GPU race on it.
-constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;  // 16 MiB
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
-
-namespace {
-std::mutex g_noalloc_mutex;
-void *g_noalloc_ptr[kMaxDevices] = {};  // device address of the array, per device ordinal
-}  // namespace
-
-size_t noalloc_scratch_bytes() { return kNoAllocScratchBytes; }
-
-// Set-up on the current device: the array's host-side name is only a
-// stand-in, so its device address is looked up with the device current.  The
-// first call on a device does this (it should come before any stream
-// capture); later calls whose stream is not capturing look it up again, so a
-// device reset (which gives the array a new address) leaves no stale pointer.
-static void *noalloc_scratch_address(cudaStream_t s) {
-  int dev = 0;
-  RCHOL_CUDA(cudaGetDevice(&dev));
-  RCHOL_CHECK_ARG(dev >= 0 && dev < kMaxDevices, "device ordinal out of range");
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
-    (void)cudaGetLastError();  // e.g. the legacy stream while another stream captures
-    cs = cudaStreamCaptureStatusActive;
-  }
-  std::lock_guard<std::mutex> guard(g_noalloc_mutex);
-  if (!g_noalloc_ptr[dev] || cs == cudaStreamCaptureStatusNone) {
-    void *p = nullptr;
-    RCHOL_CUDA(cudaGetSymbolAddress(&p, g_noalloc_scratch));
-    g_noalloc_ptr[dev] = p;
-  }
-  return g_noalloc_ptr[dev];
-}
-
-void precond_noalloc(const rchol_factor_s &F, const double *r, double *z, cudaStream_t s) {
-  const int64_t n = F.n;
-  const bool fp32 = F.precision == RCHOL_PREC_FP32;
-  const size_t vsz = fp32 ? 4 : 8;
-  const size_t acc_bytes = al16((size_t)n * vsz);
-  if (2 * acc_bytes > kNoAllocScratchBytes)
-    throw Error(RCHOL_ERR_INVALID, "n = " + std::to_string(n) + " needs " + std::to_string(2 * acc_bytes) +
-                                       " bytes of scratch; the allocation-free entry point has " +
-                                       std::to_string(kNoAllocScratchBytes) + " (n <= " +
-                                       std::to_string(kNoAllocScratchBytes / (2 * vsz)) + " for this precision)");
-  unsigned char *base = static_cast<unsigned char *>(noalloc_scratch_address(s));
-  const SolvePlan &P = *F.plan;
-  if (fp32) {
-    float *acc = reinterpret_cast<float *>(base);
-    float *y = reinterpret_cast<float *>(base + acc_bytes);
-    launch_streams<float, double, float>(P, false, r, y, acc, s);
-    launch_streams<float, float, double>(P, true, y, z, acc, s);
-  } else {
-    double *acc = reinterpret_cast<double *>(base);
-    double *y = reinterpret_cast<double *>(base + acc_bytes);
-    launch_streams<double, double, double>(P, false, r, y, acc, s);
-    launch_streams<double, double, double>(P, true, y, z, acc, s);
   }
 }
 
