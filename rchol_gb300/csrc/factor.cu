@@ -5,20 +5,23 @@
 // random_sampling0 (:643-729) and coalesce (:358-387).
 //
 // Schedule.  The nested-dissection tree is processed one depth at a time,
-// leaves first.  One warp owns one tree node and eliminates its columns in
-// order; nodes of the same depth are independent (a fill edge never joins two
-// sibling subtrees), so a launch covers every node of a depth.
+// leaves first.  One thread block of four warps (one warp at depths with very
+// many nodes) owns one tree node and eliminates its columns in order; nodes of
+// the same depth are independent (a fill edge never joins two sibling
+// subtrees), so a launch covers every node of a depth.
 //
 // Column store.  Every column c owns a slab of fill records {row, source, w}
 // in HBM (capacity fcap[c]).  Eliminating column j appends each sampled edge
 // to the slab of its smaller endpoint with one atomicAdd on that column's
 // counter -- the same store serves node-internal fill (the reference's
 // gsl_spmatrix_set) and fill deferred to an ancestor separator (its sep_edge
-// lists).  A slab that would overflow sets a flag; the host then enlarges the
-// slabs that overflowed and runs the factorization again, which gives the
-// same result because nothing depends on timing.
+// lists).  Records past a slab's capacity go to a common pool, linked per
+// column.  If the pool runs out or a column is wider than the buffers, a flag
+// is set; the host then enlarges the slabs that overflowed and runs the
+// factorization again, which gives the same result because nothing depends on
+// timing.
 //
-// Per column (one warp, shared memory only):
+// Per column (shared memory only):
 //   1. gather the initial entries (CSR row c of the upper extended Laplacian,
 //      minus the diagonal and negative ground edges) and the fill records;
 //   2. sort by (row, source) and sum duplicate rows left to right;
@@ -49,6 +52,14 @@ struct FillRec {
 };
 static_assert(sizeof(FillRec) == 16, "FillRec layout");
 
+// A record past its column's slab; next: 1 + the column's record pushed before it.
+struct PoolRec {
+  uint32_t row, src;
+  double w;
+  uint32_t next, pad_;
+};
+static_assert(sizeof(PoolRec) == 24, "PoolRec layout");
+
 enum { FLAG_FILL = 0, FLAG_WIDTH = 1, FLAG_GCAP = 2, FLAG_SINGULAR = 3, NFLAGS = 4 };
 
 struct ElimArgs {
@@ -64,6 +75,10 @@ struct ElimArgs {
   const uint32_t *fcap;
   const int64_t *fbase;
   FillRec *frec;
+  PoolRec *pool;
+  uint32_t *pool_top;        // records taken
+  uint32_t pool_cap;
+  uint32_t *head;            // per column: 1 + its last record in the pool
   int64_t *gstart;
   uint32_t *gcnt;
   int32_t *grow;
@@ -117,6 +132,37 @@ __device__ __forceinline__ uint64_t wkey(double w) {
   uint64_t b = (uint64_t)__double_as_longlong(w);
   if (b == 0x8000000000000000ull) b = 0;
   return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+}
+
+// Record s of column t.
+__device__ __forceinline__ void put_record(const ElimArgs &a, uint32_t t, uint32_t s, uint32_t cap, int64_t fb,
+                                           uint32_t row, uint32_t src, double w) {
+  if (s < cap) {
+    a.frec[fb + s] = FillRec{row, src, w};
+    return;
+  }
+  const uint32_t k = atomicAdd(a.pool_top, 1u);
+  if (k >= a.pool_cap) {
+    atomicOr(&a.flags[FLAG_FILL], 1);
+    return;
+  }
+  a.pool[k] = PoolRec{row, src, w, atomicExch(&a.head[t], k + 1u), 0u};
+}
+
+// The records of column c past its slab, one after another into key / val
+// at positions [at, most); one thread.  If the pool ran out there are fewer
+// (the run is repeated): the rest gets weight 0 to the ground vertex.
+__device__ __forceinline__ void read_pool(const ElimArgs &a, int64_t c, uint64_t *key, double *val, int at, int most) {
+  for (uint32_t k = __ldcg(&a.head[c]); k && at < most; ++at) {
+    const PoolRec *r = a.pool + (k - 1u);
+    key[at] = ((uint64_t)__ldcg(&r->row) << 32) | __ldcg(&r->src);
+    val[at] = __ldcg(&r->w);
+    k = __ldcg(&r->next);
+  }
+  for (; at < most; ++at) {
+    key[at] = ((uint64_t)(a.next - 1) << 32) | (0xffffffffu - (uint32_t)at);
+    val[at] = 0.0;
+  }
 }
 
 constexpr unsigned GCHUNK = 256;  // entries of G a warp reserves at a time
@@ -298,8 +344,7 @@ __global__ void eliminate_kernel(ElimArgs a) {
         nx_v = a.lv[r1 + lane];
       }
     }
-    uint32_t nfill = __ldcg(&a.fcnt[c]);
-    if (nfill > cap) nfill = cap;  // overflow already flagged by the writer
+    const uint32_t nall = __ldcg(&a.fcnt[c]), nfill = min(nall, cap);
     int ninit = 0;
     // initial entries: count kept ones with a ballot per 32-wide chunk
     for (int64_t k0 = r0; k0 < r1; k0 += 32) {
@@ -320,7 +365,7 @@ __global__ void eliminate_kernel(ElimArgs a) {
       }
       ninit += __popc(bal);
     }
-    int total = ninit + (int)nfill;
+    int total = ninit + (int)nall;
     if (total > E) {
       if (lane == 0) atomicMax(&a.flags[FLAG_WIDTH], total);
       total = 0;  // skip the column; the host retries with wider buffers
@@ -338,6 +383,7 @@ __global__ void eliminate_kernel(ElimArgs a) {
         aval[ninit + f1] = __hiloint2double((int)q1.w, (int)q1.z);
       }
     }
+    if (nall > cap && total && lane == 0) read_pool(a, c, akey, aval, ninit + (int)cap, total);
     __syncwarp();
     // ---- 2. sort by (row, source) and merge --------------------------------
     if (total <= 32) {
@@ -479,14 +525,8 @@ __global__ void eliminate_kernel(ElimArgs a) {
       const uint32_t t0 = min(ri0, rk0), x0 = max(ri0, rk0), t1 = min(ri1, rk1), x1 = max(ri1, rk1);
       const uint32_t s0 = e0 ? atomicAdd(&a.fcnt[t0], 1u) : 0u;
       const uint32_t s1 = e1 ? atomicAdd(&a.fcnt[t1], 1u) : 0u;
-      if (e0) {
-        if (s0 < a.fcap[t0]) a.frec[a.fbase[t0] + s0] = FillRec{x0, (uint32_t)c + 1u, w0};
-        else atomicOr(&a.flags[FLAG_FILL], 1);
-      }
-      if (e1) {
-        if (s1 < a.fcap[t1]) a.frec[a.fbase[t1] + s1] = FillRec{x1, (uint32_t)c + 1u, w1};
-        else atomicOr(&a.flags[FLAG_FILL], 1);
-      }
+      if (e0) put_record(a, t0, s0, a.fcap[t0], a.fbase[t0], x0, (uint32_t)c + 1u, w0);
+      if (e1) put_record(a, t1, s1, a.fcap[t1], a.fbase[t1], x1, (uint32_t)c + 1u, w1);
     }
     // ---- 5. column of G -------------------------------------------------------
     if (c != ground) {
@@ -526,6 +566,345 @@ __global__ void eliminate_kernel(ElimArgs a) {
     }
     __syncwarp();
   }
+}
+
+// ---- one thread block per node -----------------------------------------------
+//
+// The same column, step for step and bit for bit, by four warps.  A column is
+// a chain of dependent steps (two sorts, the duplicate sums, a prefix sum, the
+// searches), so what counts is the latency of each, and what can leave the
+// chain:
+//   * both rank sorts split the keys over the threads of a record;
+//   * the uniforms, the weights (an FP64 division), the square root and the
+//     reciprocal of the pivot are made by other warps than the scan and the
+//     searches (an FP64 instruction holds a quarter of an SM for 64 cycles);
+//   * the next column's slab and matrix row are read during this column;
+//     only this column's own records for it are added at the end, from
+//     shared memory;
+//   * a record's place comes back from its atomicAdd while the next column
+//     is being sorted, and is written then.
+// 80^3 log-normal, 128 subdomains, one run over all columns: 9.8 us per root
+// column with one warp.
+constexpr int EB = 128;  // threads
+
+// Ranks of n <= 128 records (unique keys) over the block: every record has
+// EB / np threads, each counting the keys before it in its share.
+template <typename Before>
+__device__ __forceinline__ int block_rank(int n, int *part, Before before) {
+  const int tid = threadIdx.x;
+  const int np = n <= 32 ? 32 : n <= 64 ? 64 : 128, ways = EB / np;
+  const int r = tid & (np - 1), q = tid / np;
+  const int len = (n + ways - 1) / ways, f0 = q * len, f1 = min(n, f0 + len);
+  int c = 0;
+  if (r < n) {
+    int f = f0;
+    for (; f + 4 <= f1; f += 4) c += before(f, r) + before(f + 1, r) + before(f + 2, r) + before(f + 3, r);
+    for (; f < f1; ++f) c += before(f, r);
+  }
+  part[tid] = c;
+  __syncthreads();
+  if (tid >= n) return -1;
+  int rank = 0;
+  for (int w = 0; w < ways; ++w) rank += part[tid + w * np];
+  return rank;
+}
+
+__global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int part[EB];
+  __shared__ int s_n[2];  // records in the input buffers
+  __shared__ unsigned long long s_gs;
+  __shared__ double s_sq, s_inv;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int E = a.emax;
+  uint64_t *akey = reinterpret_cast<uint64_t *>(smem_raw);
+  double *aval = reinterpret_cast<double *>(akey + E);
+  uint64_t *bkey = reinterpret_cast<uint64_t *>(aval + E);
+  double *bval = reinterpret_cast<double *>(bkey + E);
+  double *cs = bval + E;
+  uint64_t *ikey = reinterpret_cast<uint64_t *>(cs + E);  // [2][E] input buffers
+  double *ival = reinterpret_cast<double *>(ikey + 2 * E);
+  double *uni = ival + 2 * E, *wv = uni + E;
+  uint32_t *kk = reinterpret_cast<uint32_t *>(wv + E);
+  const int64_t ground = a.next - 1;
+  const int64_t cb = a.node_begin[blockIdx.x], ce = a.node_end[blockIdx.x];
+  // the matrix row of column c into an input buffer from position `at` on; one warp
+  auto put_row = [&](int64_t c, int64_t r0, int64_t r1, int32_t col0, double v0, uint64_t *key, double *val, int at) {
+    for (int64_t k0 = r0; k0 < r1; k0 += 32) {
+      const int64_t k = k0 + lane;
+      bool keep = false;
+      int32_t col = 0;
+      double v = 0.0;
+      if (k < r1) {
+        col = k0 == r0 ? col0 : a.lci[k];
+        v = k0 == r0 ? v0 : a.lv[k];
+        keep = (col != c) && !(col == ground && v < 0.0 && c != ground);
+      }
+      const unsigned bal = __ballot_sync(0xffffffffu, keep);
+      const int pos = at + __popc(bal & ((1u << lane) - 1u));
+      if (keep && pos < E) {
+        key[pos] = ((uint64_t)(uint32_t)col << 32);
+        val[pos] = v;
+      }
+      at += __popc(bal);
+    }
+    return at;
+  };
+  auto put_slab = [&](uint32_t f, const uint4 q, uint64_t *key, double *val) {
+    key[f] = ((uint64_t)q.x << 32) | q.y;
+    val[f] = __hiloint2double((int)q.w, (int)q.z);
+  };
+  // first column: everything read here
+  {
+    const uint32_t nall = __ldcg(&a.fcnt[cb]), cap = a.fcap[cb], nslab = min(min(nall, cap), (uint32_t)E);
+    for (uint32_t f = tid; f < nslab; f += EB)
+      put_slab(f, __ldcg(reinterpret_cast<const uint4 *>(a.frec + a.fbase[cb] + f)), ikey, ival);
+    if (nall > cap && tid == 0) read_pool(a, cb, ikey, ival, (int)cap, min((int)nall, E));
+    if (warp == 3) {
+      const int64_t r0 = a.lrp[cb], r1 = a.lrp[cb + 1];
+      int32_t col = 0;
+      double v = 0.0;
+      if (r0 + lane < r1) col = a.lci[r0 + lane], v = a.lv[r0 + lane];
+      const int n = put_row(cb, r0, r1, col, v, ikey, ival, (int)nall);
+      if (lane == 0) s_n[0] = n;
+    }
+  }
+  // static facts of the next column, loaded a column before they are needed
+  uint32_t nx_cap = 0;
+  int64_t nx_fb = 0, nx_r0 = 0, nx_r1 = 0;
+  auto facts = [&](int64_t c) {
+    if (c < ce) {
+      nx_cap = a.fcap[c];
+      nx_fb = a.fbase[c];
+      if (warp == 3) nx_r0 = a.lrp[c], nx_r1 = a.lrp[c + 1];
+    }
+  };
+  facts(cb + 1);
+  unsigned long long gcur = 0, gend = 0;  // thread 32: this block's reserved run of G
+  // a record whose place is still on its way
+  bool pend = false;
+  uint32_t p_t = 0, p_s = 0, p_cap = 0, p_x = 0, p_src = 0;
+  int64_t p_fb = 0;
+  double p_w = 0.0;
+  __syncthreads();
+  for (int64_t c = cb; c < ce; ++c) {
+    const int cur = (int)(c - cb) & 1;
+    uint64_t *ckey = ikey + cur * E, *nkey = ikey + (cur ^ 1) * E;
+    double *cval = ival + cur * E, *nval = ival + (cur ^ 1) * E;
+    int n = s_n[cur];
+    if (n > E) {
+      if (tid == 0) atomicMax(&a.flags[FLAG_WIDTH], n);
+      n = 0;  // skip the column; the host retries with wider buffers
+    }
+    // ---- sort by (row, source); the last column's records are written -------
+    if (pend) put_record(a, p_t, p_s, p_cap, p_fb, p_x, p_src, p_w);
+    pend = false;
+    if (n <= EB) {
+      const uint64_t mine = (tid & ((n <= 32 ? 32 : n <= 64 ? 64 : 128) - 1)) < n
+                                ? ckey[tid & ((n <= 32 ? 32 : n <= 64 ? 64 : 128) - 1)]
+                                : 0;
+      const int rank = block_rank(n, part, [&](int f, int) { return (int)(ckey[f] < mine); });
+      if (rank >= 0) {
+        bkey[rank] = mine;
+        bval[rank] = cval[tid];
+      }
+    } else {
+      if (warp == 0)
+        warp_bitonic_sort(ckey, cval, n, [](uint64_t ka, double, uint64_t kb, double) { return ka < kb; });
+      __syncthreads();
+      for (int e = tid; e < n; e += EB) bkey[e] = ckey[e], bval[e] = cval[e];
+    }
+    __syncthreads();
+    // every record of the columns before c is in place: the next column's count
+    const bool more = c + 1 < ce;
+    const uint32_t nx_all = more ? __ldcg(&a.fcnt[c + 1]) : 0u;
+    const uint32_t cap1 = nx_cap;
+    const int64_t fb1 = nx_fb, r01 = nx_r0, r11 = nx_r1;
+    int32_t row_col = 0;
+    double row_v = 0.0;
+    if (more && warp == 3 && r01 + lane < r11) row_col = a.lci[r01 + lane], row_v = a.lv[r01 + lane];
+    facts(c + 2);
+    // ---- duplicates: a row's first record sums the others left to right -----
+    int m = 0;
+    uint64_t *wk = reinterpret_cast<uint64_t *>(cs);  // cs is free until the prefix sum
+    for (int e0 = 0; e0 < n; e0 += EB) {
+      const int e = e0 + tid;
+      int before = m;
+#pragma unroll
+      for (int w = 0; w < EB / 32; ++w) {  // heads of the block's four chunks
+        const int x = e0 + 32 * w + lane;
+        const bool h = x < n && (x == 0 || (uint32_t)(bkey[x - 1] >> 32) != (uint32_t)(bkey[x] >> 32));
+        const unsigned bal = __ballot_sync(0xffffffffu, h);
+        if (w < warp) before += __popc(bal);
+        else if (w == warp) before += __popc(bal & ((1u << lane) - 1u));
+        m += __popc(bal);
+      }
+      if (e < n) {
+        const uint32_t row = (uint32_t)(bkey[e] >> 32);
+        if (e == 0 || (uint32_t)(bkey[e - 1] >> 32) != row) {
+          double s = bval[e];
+          for (int f = e + 1; f < n && (uint32_t)(bkey[f] >> 32) == row; ++f) s = __dadd_rn(s, bval[f]);
+          akey[before] = row;  // rows ascending
+          aval[before] = s;
+          wk[before] = wkey(s);
+        }
+      }
+    }
+    __syncthreads();
+    // ---- sort by (weight, row) ---------------------------------------------
+    if (m <= EB) {
+      const int np = m <= 32 ? 32 : m <= 64 ? 64 : 128, r = tid & (np - 1);
+      const uint64_t mw = r < m ? wk[r] : 0;
+      const uint32_t mr = r < m ? (uint32_t)akey[r] : 0;
+      const int rank = block_rank(m, part, [&](int f, int) {
+        const uint64_t wf = wk[f];
+        return (int)((wf < mw) | ((wf == mw) & ((uint32_t)akey[f] < mr)));
+      });
+      if (rank >= 0) {
+        bkey[rank] = mr;
+        bval[rank] = aval[tid];
+      }
+    } else {
+      for (int e = tid; e < m; e += EB) bkey[e] = (uint32_t)akey[e], bval[e] = aval[e];
+      __syncthreads();
+      if (warp == 0)
+        warp_bitonic_sort(bkey, bval, m, [](uint64_t ra, double wa, uint64_t rb, double wb) {
+          return wless(wa, (uint32_t)ra, wb, (uint32_t)rb);
+        });
+    }
+    // the next column's slab, loaded while this one is scanned and sampled
+    const uint32_t nslab = min(min(nx_all, cap1), (uint32_t)E);
+    uint4 pre = make_uint4(0u, 0u, 0u, 0u);
+    if ((uint32_t)tid < nslab) pre = __ldcg(reinterpret_cast<const uint4 *>(a.frec + fb1 + tid));
+    __syncthreads();
+    // ---- prefix sum (warp 0), uniforms (the others), place in G -------------
+    const bool hasg = m > 0 && (int64_t)(uint32_t)akey[m - 1] == ground;
+    const int cnt = 1 + m - (hasg ? 1 : 0);
+    if (warp == 0) {
+      double carry = 0.0;
+      for (int e0 = 0; e0 < m; e0 += 64) {
+        const int ea = e0 + lane, eb = ea + 32;
+        const bool two = e0 + 32 < m;
+        double va = (ea < m) ? bval[ea] : 0.0, vb = (two && eb < m) ? bval[eb] : 0.0;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const double ta = __shfl_up_sync(0xffffffffu, va, d);
+          if (lane >= d) va = __dadd_rn(ta, va);
+          if (two) {
+            const double tb = __shfl_up_sync(0xffffffffu, vb, d);
+            if (lane >= d) vb = __dadd_rn(tb, vb);
+          }
+        }
+        const double outa = __dadd_rn(carry, va);
+        if (ea < m) cs[ea] = outa;
+        carry = __shfl_sync(0xffffffffu, outa, min(31, m - 1 - e0));
+        if (two) {
+          const double outb = __dadd_rn(carry, vb);
+          if (eb < m) cs[eb] = outb;
+          carry = __shfl_sync(0xffffffffu, outb, min(31, m - 1 - e0 - 32));
+        }
+      }
+    } else {
+      for (int i = tid - 32; i < m - 1; i += EB - 32) uni[i] = uniform53(a.seed, (uint64_t)c, (uint32_t)i);
+      if (tid == 32 && c != ground) {
+        if (gcur + (unsigned)cnt > gend) {
+          const unsigned long long take = max((unsigned)cnt, GCHUNK);
+          gcur = atomicAdd(a.gtop, take);
+          gend = gcur + take;
+        }
+        s_gs = gcur;
+        gcur += (unsigned)cnt;
+      }
+    }
+    __syncthreads();
+    const double csum = m ? cs[m - 1] : 0.0;
+    // ---- sample: even warps search, odd warps make the weights --------------
+    for (int i0 = (warp >> 1) * 32; i0 < m - 1; i0 += EB / 2) {
+      const int i = i0 + lane;
+      if (i >= m - 1) continue;
+      const double tar = cs[i], span = __dsub_rn(csum, tar);
+      if (!(warp & 1)) {
+        const uint64_t r = wkey(__dadd_rn(__dmul_rn(uni[i], span), tar));
+        int lo = i, hi = m;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (wkey(cs[mid]) < r) lo = mid + 1;
+          else hi = mid;
+        }
+        kk[i] = (uint32_t)(lo < m ? lo : m - 1);
+      } else {
+        wv[i] = __ddiv_rn(__dmul_rn(bval[i], span), csum);
+      }
+    }
+    if (warp == 2 && c != ground) {
+      const double sq = __dsqrt_rn(csum);
+      if (lane == 0) {
+        s_sq = sq;
+        a.diag[c] = csum;
+        if (!(csum > 0.0)) atomicOr(&a.flags[FLAG_SINGULAR], 1);
+      }
+    }
+    if (warp == 3) {
+      if (c != ground) {
+        const double inv = __ddiv_rn(1.0, csum);
+        if (lane == 0) s_inv = inv;
+      } else if (lane == 0) {
+        a.diag[c] = csum;
+      }
+      int total = 0;
+      if (more) total = put_row(c + 1, r01, r11, row_col, row_v, nkey, nval, (int)nx_all);
+      if (lane == 0) s_n[cur ^ 1] = total;
+    }
+    if ((uint32_t)tid < nslab) put_slab((uint32_t)tid, pre, nkey, nval);
+    for (uint32_t f = tid + EB; f < nslab; f += EB)
+      put_slab(f, __ldcg(reinterpret_cast<const uint4 *>(a.frec + fb1 + f)), nkey, nval);
+    if (nx_all > cap1 && tid == 0) read_pool(a, c + 1, nkey, nval, (int)cap1, min((int)nx_all, E));
+    __syncthreads();
+    // ---- records of the sampled edges ---------------------------------------
+    for (int i = tid; i < m - 1; i += EB) {
+      const int k = (int)kk[i];
+      if (k == i) continue;
+      const uint32_t ri = (uint32_t)bkey[i], rk = (uint32_t)bkey[k], t = min(ri, rk), x = max(ri, rk);
+      const double w = wv[i];
+      if (more && (int64_t)t == c + 1) {
+        const int at = atomicAdd(&s_n[cur ^ 1], 1);
+        if (at < E) {
+          nkey[at] = ((uint64_t)x << 32) | ((uint32_t)c + 1u);
+          nval[at] = w;
+        }
+        continue;
+      }
+      const uint32_t s = atomicAdd(&a.fcnt[t], 1u), cap = a.fcap[t];
+      const int64_t fb = a.fbase[t];
+      if (i + EB < m - 1) {  // another edge follows: written now
+        put_record(a, t, s, cap, fb, x, (uint32_t)c + 1u, w);
+      } else {
+        pend = true;
+        p_t = t, p_s = s, p_cap = cap, p_fb = fb, p_x = x, p_src = (uint32_t)c + 1u, p_w = w;
+      }
+    }
+    // ---- column of G ----------------------------------------------------------
+    if (c != ground) {
+      const unsigned long long gs = s_gs;
+      if ((int64_t)(gs + cnt) > a.gcap) {
+        if (tid == 0) atomicOr(&a.flags[FLAG_GCAP], 1);
+      } else {
+        const double sq = s_sq, inv = s_inv;
+        if (tid == EB - 1) {
+          a.gstart[c] = (int64_t)gs;
+          a.gcnt[c] = (uint32_t)cnt;
+          a.grow[gs] = (int32_t)c;
+          a.gval[gs] = sq;
+        }
+        for (int e = EB - 1 - tid; e < cnt - 1; e += EB) {
+          a.grow[gs + 1 + e] = (int32_t)(uint32_t)akey[e];
+          a.gval[gs + 1 + e] = __dmul_rn(-__dmul_rn(aval[e], inv), sq);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (pend) put_record(a, p_t, p_s, p_cap, p_fb, p_x, p_src, p_w);
 }
 
 // ---- CSR assembly ----------------------------------------------------------
@@ -617,15 +996,24 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
   const size_t smem_limit = prop.sharedMemPerBlockOptin;
   RCHOL_CUDA(cudaFuncSetAttribute(eliminate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_limit));
+  const size_t block_limit = smem_limit - 2048;  // beside the static arrays
+  RCHOL_CUDA(cudaFuncSetAttribute(eliminate_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)block_limit));
+  const int64_t pool_cap = std::max<int64_t>(1 << 16, next / 4);
 
   DevBuf<double> diag(next);
   DevBuf<int> flags(NFLAGS);
+  int widest = 0;  // the widest column that did not fit a buffer so far
   for (int attempt = 0; attempt < 12; ++attempt) {
     std::vector<int64_t> base(next + 1, 0);
     for (int64_t c = 0; c < next; ++c) base[c + 1] = base[c] + cap[c];
     DevBuf<uint32_t> fcnt(next), fcap(next);
     DevBuf<int64_t> fbase(next);
     DevBuf<FillRec> frec(std::max<int64_t>(base[next], 1));
+    DevBuf<PoolRec> pool(pool_cap);
+    DevBuf<uint32_t> head(next), pool_top(1);
+    RCHOL_CUDA(cudaMemsetAsync(head.p, 0, head.bytes(), s));
+    RCHOL_CUDA(cudaMemsetAsync(pool_top.p, 0, pool_top.bytes(), s));
     DevBuf<int64_t> gstart(next);
     DevBuf<uint32_t> gcnt(next);
     DevBuf<int32_t> grow(gcap);
@@ -649,6 +1037,10 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
     args.fcap = fcap.p;
     args.fbase = fbase.p;
     args.frec = frec.p;
+    args.pool = pool.p;
+    args.pool_top = pool_top.p;
+    args.pool_cap = (uint32_t)pool_cap;
+    args.head = head.p;
     args.gstart = gstart.p;
     args.gcnt = gcnt.p;
     args.grow = grow.p;
@@ -661,7 +1053,7 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
     std::vector<DevBuf<int64_t>> keep;
     for (int depth = maxdepth; depth >= 1; --depth) {
       std::vector<int64_t> nb, ne;
-      int width = 32;
+      int width = std::max(32, widest);
       for (auto &nd : nodes) {
         if (nd.depth != depth || nd.end <= nd.begin) continue;
         nb.push_back(nd.begin);
@@ -670,7 +1062,23 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
           width = std::max(width, initdeg[c] + (int)cap[c]);
       }
       if (nb.empty()) continue;
-      int emax = pow2_at_least(width);
+      // four warps per node unless the nodes alone fill the GPU several times
+      const size_t block_bytes = (size_t)std::max(256, pow2_at_least(width)) * 96;
+      if ((int64_t)nb.size() <= 8 * (int64_t)prop.multiProcessorCount && block_bytes <= block_limit) {
+        keep.emplace_back(nb.size());
+        keep.back().upload(nb.data(), nb.size(), s);
+        keep.emplace_back(ne.size());
+        keep.back().upload(ne.data(), ne.size(), s);
+        args.node_begin = keep[keep.size() - 2].p;
+        args.node_end = keep.back().p;
+        args.num_nodes = (int)nb.size();
+        args.emax = std::max(256, pow2_at_least(width));
+        args.gscratch = nullptr;
+        eliminate_block_kernel<<<(unsigned)nb.size(), EB, block_bytes, s>>>(args);
+        RCHOL_CUDA(cudaGetLastError());
+        continue;
+      }
+      int emax = pow2_at_least(std::max(width, 128));
       size_t per_warp = (size_t)emax * 40;
       const bool in_smem = per_warp <= smem_limit;
       int wpb = in_smem ? (int)std::min<size_t>(4, smem_limit / per_warp) : 1;
@@ -694,6 +1102,7 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
     flags.download(hflags, NFLAGS, s);
     RCHOL_CUDA(cudaStreamSynchronize(s));
     if (hflags[FLAG_FILL] || hflags[FLAG_WIDTH]) {
+      widest = std::max(widest, hflags[FLAG_WIDTH]);
       // Counts past an overflow are lower bounds (truncated columns sample
       // less fill into the columns after them).  Overflowing columns grow to
       // twice their count.  The other columns of an overflowing depth grow
