@@ -33,6 +33,7 @@
 // (team_k_kernel).
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -61,35 +62,34 @@ __host__ __device__ inline int tri_col_off(int c, bool upper) {
 
 // ---- host: one piece -----------------------------------------------------------
 
-struct PieceBuild {
+struct PieceBuild {  // blocks [s0, s1) of a piece
+  int64_t s0 = 0, s1 = 0;
   std::vector<unsigned char> bytes;  // block records, processing order
-  std::vector<int64_t> offs;         // nblocks + 1 relative offsets
+  std::vector<int64_t> offs;         // s1 - s0 + 1 relative offsets
   int32_t maxrec = 0;
   int64_t sparse = 0;
 };
 
 // Exact inverse of a 32x32 triangular block (rows/cols >= nr are identity).
+// Entry (i, j) is -(sum over k ascending of T[i][k] X[k][j]) / T[i][i]; the
+// sums of a row run side by side over j, which the compiler vectorises.
 void invert_block(double T[BS][BS], bool upper, double X[BS][BS]) {
   for (int r = 0; r < BS; ++r)
     for (int c = 0; c < BS; ++c) X[r][c] = 0.0;
-  if (!upper) {
-    for (int j = 0; j < BS; ++j) {
-      X[j][j] = 1.0 / T[j][j];
-      for (int i = j + 1; i < BS; ++i) {
-        double s = 0.0;
-        for (int k = j; k < i; ++k) s += T[i][k] * X[k][j];
-        X[i][j] = -s / T[i][i];
-      }
+  double s[BS];
+  for (int u = 0; u < BS; ++u) {
+    const int i = upper ? BS - 1 - u : u;
+    for (int j = 0; j < BS; ++j) s[j] = 0.0;
+    if (!upper) {
+      for (int k = 0; k < i; ++k)
+        for (int j = 0; j <= k; ++j) s[j] += T[i][k] * X[k][j];
+      for (int j = 0; j < i; ++j) X[i][j] = -s[j] / T[i][i];
+    } else {
+      for (int k = i + 1; k < BS; ++k)
+        for (int j = k; j < BS; ++j) s[j] += T[i][k] * X[k][j];
+      for (int j = i + 1; j < BS; ++j) X[i][j] = -s[j] / T[i][i];
     }
-  } else {
-    for (int j = BS - 1; j >= 0; --j) {
-      X[j][j] = 1.0 / T[j][j];
-      for (int i = j - 1; i >= 0; --i) {
-        double s = 0.0;
-        for (int k = i + 1; k <= j; ++k) s += T[i][k] * X[k][j];
-        X[i][j] = -s / T[i][i];
-      }
-    }
+    X[i][i] = 1.0 / T[i][i];
   }
 }
 
@@ -160,7 +160,7 @@ void build_team_piece(const std::vector<int64_t> &rp, const std::vector<int32_t>
   maxchunk = 0;
   double T[BS][BS], X[BS][BS];
   std::vector<std::pair<uint32_t, double>> nearl[BS], farl[BS];
-  for (int64_t s = 0; s < nb; ++s) {
+  for (int64_t s = P.s0; s < P.s1; ++s) {
     const int64_t bi = upper ? nb - 1 - s : s;
     const int64_t row0 = bi * BS;
     const int nr = (int)std::min<int64_t>(BS, R - row0);
@@ -668,7 +668,7 @@ void build_w2_piece(const std::vector<int64_t> &rp, const std::vector<int32_t> &
   double T[BS][BS], X[BS][BS];
   std::vector<uint32_t> cols[BS];
   std::vector<double> vals[BS];
-  for (int64_t s = 0; s < nb; ++s) {
+  for (int64_t s = P.s0; s < P.s1; ++s) {
     const int64_t bi = upper ? nb - 1 - s : s;
     const int64_t row0 = bi * BS;
     const int nr = (int)std::min<int64_t>(BS, R - row0);
@@ -812,7 +812,7 @@ void build_pipe_piece(const std::vector<int64_t> &rp, const std::vector<int32_t>
   maxchunk = 0;
   double T[BS][BS], X[BS][BS], N1[BS][BS], N2[BS][BS];
   std::vector<std::pair<uint32_t, double>> lf[BS];
-  for (int64_t s = 0; s < nb; ++s) {
+  for (int64_t s = P.s0; s < P.s1; ++s) {
     const int64_t bi = upper ? nb - 1 - s : s;
     const int64_t row0 = bi * BS;
     const int nr = (int)std::min<int64_t>(BS, R - row0);
@@ -862,19 +862,23 @@ void build_pipe_piece(const std::vector<int64_t> &rp, const std::vector<int32_t>
     std::memcpy(p, hdr, sizeof(hdr));
     put_tinv(p + L.o_tinv, vsz, X, nr, upper);
     // P = T^-1 N1, Q = T^-1 N2 (rows and columns beyond the block's rows are zero)
-    for (int r = 0; r < BS; ++r)
-      for (int c = 0; c < BS; ++c) {
-        double pr = 0.0, qr = 0.0;
-        if (r < nr)
-          for (int k = 0; k < nr; ++k) {
-            const double t = X[r][k];
-            if (t == 0.0) continue;
-            pr += t * N1[k][c];
-            qr += t * N2[k][c];
+    // (terms in ascending k; the columns of a row side by side)
+    for (int r = 0; r < BS; ++r) {
+      double pr[BS] = {}, qr[BS] = {};
+      if (r < nr)
+        for (int k = 0; k < nr; ++k) {
+          const double t = X[r][k];
+          if (t == 0.0) continue;
+          for (int c = 0; c < BS; ++c) {
+            pr[c] += t * N1[k][c];
+            qr[c] += t * N2[k][c];
           }
-        put_val(p + L.o_p, vsz, (size_t)r * stride + c, pr);
-        put_val(p + L.o_q, vsz, (size_t)r * stride + c, qr);
+        }
+      for (int c = 0; c < BS; ++c) {
+        put_val(p + L.o_p, vsz, (size_t)r * stride + c, pr[c]);
+        put_val(p + L.o_q, vsz, (size_t)r * stride + c, qr[c]);
       }
+    }
     std::memcpy(p + L.o_crow, crow, sizeof(crow));
     // chunk c holds row r's far entries crow[r]*clen.. in column order; within
     // each warp's 32 chunks the entries of one step are picked greedily so that
@@ -1867,51 +1871,70 @@ static void build_dir_streams(const std::vector<int64_t> &rp, const std::vector<
         }
     }
   }, 1 << 14);
-  // block records, the largest pieces first (they take the longest)
-  std::vector<PieceBuild> built(np);
-  std::vector<int32_t> chunks(np, 0);
-  std::vector<int> by_size(np);
-  for (int k = 0; k < np; ++k) by_size[k] = k;
-  std::stable_sort(by_size.begin(), by_size.end(),
-                   [&](int x, int y) { return pieces[x].e - pieces[x].b > pieces[y].e - pieces[y].b; });
-  parallel_for(np, [&](int64_t k0, int64_t k1) {
-    for (int64_t kk = k0; kk < k1; ++kk) {
-      const int k = by_size[kk];
-      const Piece &pc = pieces[k];
+  // Block records, in runs of up to kBuildRun blocks: the records of a piece
+  // do not depend on one another, and the root's alone would keep one thread
+  // busy while the others wait (80^3, 128 subdomains: 43 ms of a direction's
+  // 64 with one task per piece).
+  constexpr int64_t kBuildRun = 16;
+  std::vector<PieceBuild> built;
+  std::vector<int> run_piece;
+  for (int k = 0; k < np; ++k) {
+    const int64_t nb = (pieces[k].e - pieces[k].b + BS - 1) / BS;
+    for (int64_t s0 = 0; s0 < nb; s0 += kBuildRun) {
+      built.emplace_back();
+      built.back().s0 = s0;
+      built.back().s1 = std::min(nb, s0 + kBuildRun);
+      run_piece.push_back(k);
+    }
+  }
+  const int64_t nruns = (int64_t)built.size();
+  std::vector<int32_t> chunks(nruns, 0);
+  // one run at a time per thread, from the top of the tree with its long rows
+  std::atomic<int64_t> next_run{0};
+  parallel_for(host_threads(), [&](int64_t, int64_t) {
+    for (int64_t i; (i = next_run.fetch_add(1)) < nruns;) {
+      const int64_t r = upper ? i : nruns - 1 - i;
+      const Piece &pc = pieces[run_piece[r]];
       if (pc.fmt == FMT_WARP) {
         int64_t reach = 0;
-        build_w2_piece(rp, ci, v, pc.b, pc.e, upper, vsz, built[k], reach);
+        build_w2_piece(rp, ci, v, pc.b, pc.e, upper, vsz, built[r], reach);
         if (reach + BS >= pc.window && pc.window < pc.e - pc.b)
           throw Error(RCHOL_ERR_INTERNAL, "warp-format window shorter than the piece's reach");
       } else if (pc.fmt == FMT_PIPE) {
-        build_pipe_piece(rp, ci, v, pc.b, pc.e, upper, vsz, 32 * (pc.warps - kPipeRoleWarps), built[k], chunks[k]);
+        build_pipe_piece(rp, ci, v, pc.b, pc.e, upper, vsz, 32 * (pc.warps - kPipeRoleWarps), built[r], chunks[r]);
       } else {
-        build_team_piece(rp, ci, v, pc.b, pc.e, upper, vsz, 32 * (pc.warps - 1), true, built[k], chunks[k]);
+        build_team_piece(rp, ci, v, pc.b, pc.e, upper, vsz, 32 * (pc.warps - 1), true, built[r], chunks[r]);
       }
     }
   }, 1);
   std::vector<NodeDesc> desc(np);
-  std::vector<int64_t> blk_off;
-  int64_t total = 0;
+  std::vector<int64_t> blk_off, run_off(nruns);
+  int64_t total = 0, run = 0;
   D.sparse_nnz = 0;
   for (int k = 0; k < np; ++k) {
     desc[k].begin = pieces[k].b;
     desc[k].rows = (int32_t)(pieces[k].e - pieces[k].b);
-    desc[k].nblocks = (int32_t)(built[k].offs.size() - 1);
+    desc[k].nblocks = (desc[k].rows + BS - 1) / BS;
     desc[k].blk0 = (int64_t)blk_off.size();
-    desc[k].maxrec = built[k].maxrec;
+    desc[k].maxrec = 0;
     desc[k].wide = desc[k].rows > 65535;
-    desc[k].maxchunk = chunks[k];
+    desc[k].maxchunk = 0;
     desc[k].pad_ = 0;
-    for (int64_t o : built[k].offs) blk_off.push_back(total + o);
-    total += (int64_t)built[k].bytes.size();
-    D.sparse_nnz += built[k].sparse;
+    for (; run < nruns && run_piece[run] == k; ++run) {
+      const PieceBuild &B = built[run];
+      desc[k].maxrec = std::max(desc[k].maxrec, B.maxrec);
+      desc[k].maxchunk = std::max(desc[k].maxchunk, chunks[run]);
+      for (int64_t j = 0; j < B.s1 - B.s0; ++j) blk_off.push_back(total + B.offs[j]);
+      run_off[run] = total;
+      total += (int64_t)B.bytes.size();
+      D.sparse_nnz += B.sparse;
+    }
+    blk_off.push_back(total);
   }
-  // every byte is written by one piece's copy: no zero fill
+  // every byte is written by one run's copy: no zero fill
   std::unique_ptr<unsigned char[]> all(new unsigned char[std::max<int64_t>(total, 1)]);
-  parallel_for(np, [&](int64_t k0, int64_t k1) {
-    for (int64_t k = k0; k < k1; ++k)
-      std::memcpy(all.get() + blk_off[desc[k].blk0], built[k].bytes.data(), built[k].bytes.size());
+  parallel_for(nruns, [&](int64_t r0, int64_t r1) {
+    for (int64_t r = r0; r < r1; ++r) std::memcpy(all.get() + run_off[r], built[r].bytes.data(), built[r].bytes.size());
   }, 1);
   built.clear();
   // stages
