@@ -5,7 +5,7 @@
 // random_sampling0 (:643-729) and coalesce (:358-387).
 //
 // Schedule.  The nested-dissection tree is processed one depth at a time,
-// leaves first.  One thread block of eight warps (one warp at depths with very
+// leaves first.  One thread block of four warps (one warp at depths with very
 // many nodes) owns one tree node and eliminates its columns in order; nodes of
 // the same depth are independent (a fill edge never joins two sibling
 // subtrees), so a launch covers every node of a depth.
@@ -570,61 +570,38 @@ __global__ void eliminate_kernel(ElimArgs a) {
 
 // ---- one thread block per node -----------------------------------------------
 //
-// The same column, step for step and bit for bit, by eight warps.  A column is
+// The same column, step for step and bit for bit, by four warps.  A column is
 // a chain of dependent steps (two sorts, the duplicate sums, a prefix sum, the
 // searches), so what counts is the latency of each, and what can leave the
 // chain:
 //   * both rank sorts split the keys over the threads of a record;
-//   * the 32-wide chunks of the prefix sum are scanned by a warp each;
-//   * searches, weights (an FP64 division), square root and reciprocal of the
-//     pivot go to different warps and, an FP64 instruction holding its quarter
-//     of the SM for 64 cycles, to different quarters; the uniforms are made
-//     with integers alone;
+//   * the uniforms, the weights (an FP64 division), the square root and the
+//     reciprocal of the pivot are made by other warps than the scan and the
+//     searches (an FP64 instruction holds a quarter of an SM for 64 cycles);
 //   * the next column's slab and matrix row are read during this column;
 //     only this column's own records for it are added at the end, from
 //     shared memory;
 //   * a record's place comes back from its atomicAdd while the next column
 //     is being sorted, and is written then.
-constexpr int EB = 256;       // threads
-constexpr int RANK_MAX = 128; // most records of the rank sorts
+// 80^3 log-normal, 128 subdomains, one run over all columns: 9.8 us per root
+// column with one warp.
+constexpr int EB = 128;  // threads
 
-// uniform53 without FP64 instructions: k / 2^53 for a 53-bit integer k is
-// exact, so its bits follow from k's leading bit.
-__device__ __forceinline__ double uniform53_bits(uint64_t seed, uint64_t v, uint32_t i) {
-  uint32_t c[4] = {i >> 1, 0u, (uint32_t)v, (uint32_t)(v >> 32)};
-  philox(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-  const uint32_t a = (i & 1) ? c[2] : c[0], b = (i & 1) ? c[3] : c[1];
-  const uint64_t k = ((uint64_t)(a >> 5) << 26) + (b >> 6);
-  if (!k) return 0.0;
-  const int lz = __clzll((long long)k);  // at least 11
-  const uint64_t mant = (k << (lz - 11)) & 0xfffffffffffffull;
-  return __longlong_as_double((long long)(((uint64_t)(1023 + 63 - lz - 53) << 52) | mant));
-}
-
-// Ranks of n <= RANK_MAX unique keys (16-byte aligned): record r has EB / np
-// threads, each counting the keys before it in its share; equal keys (weights)
-// order by place.  `mid` runs before the block meets.  Threads below n get
-// their record's rank, the others -1.
-template <typename Mid>
-__device__ __forceinline__ int block_rank(const uint64_t *key, int n, int *part, Mid mid) {
+// Ranks of n <= 128 records (unique keys) over the block: every record has
+// EB / np threads, each counting the keys before it in its share.
+template <typename Before>
+__device__ __forceinline__ int block_rank(int n, int *part, Before before) {
   const int tid = threadIdx.x;
   const int np = n <= 32 ? 32 : n <= 64 ? 64 : 128, ways = EB / np;
   const int r = tid & (np - 1), q = tid / np;
-  const int len = ((n + ways - 1) / ways + 1) & ~1, f0 = min(n, q * len), f1 = min(n, f0 + len);
+  const int len = (n + ways - 1) / ways, f0 = q * len, f1 = min(n, f0 + len);
   int c = 0;
   if (r < n) {
-    const uint64_t mine = key[r];
-    auto before = [&](uint64_t k, int f) { return (int)((k < mine) | ((k == mine) & (f < r))); };
     int f = f0;
-    for (; f + 4 <= f1; f += 4) {
-      const ulonglong2 k0 = *reinterpret_cast<const ulonglong2 *>(key + f),
-                       k1 = *reinterpret_cast<const ulonglong2 *>(key + f + 2);
-      c += before(k0.x, f) + before(k0.y, f + 1) + (before(k1.x, f + 2) + before(k1.y, f + 3));
-    }
-    for (; f < f1; ++f) c += before(key[f], f);
+    for (; f + 4 <= f1; f += 4) c += before(f, r) + before(f + 1, r) + before(f + 2, r) + before(f + 3, r);
+    for (; f < f1; ++f) c += before(f, r);
   }
   part[tid] = c;
-  mid();
   __syncthreads();
   if (tid >= n) return -1;
   int rank = 0;
@@ -638,7 +615,6 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
   __shared__ int s_n[2];  // records in the input buffers
   __shared__ unsigned long long s_gs;
   __shared__ double s_sq, s_inv;
-  __shared__ double s_last[EB / 32];  // sums of the prefix sum's chunks
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int E = a.emax;
   uint64_t *akey = reinterpret_cast<uint64_t *>(smem_raw);
@@ -684,7 +660,7 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
     for (uint32_t f = tid; f < nslab; f += EB)
       put_slab(f, __ldcg(reinterpret_cast<const uint4 *>(a.frec + a.fbase[cb] + f)), ikey, ival);
     if (nall > cap && tid == 0) read_pool(a, cb, ikey, ival, (int)cap, min((int)nall, E));
-    if (warp == 7) {
+    if (warp == 3) {
       const int64_t r0 = a.lrp[cb], r1 = a.lrp[cb + 1];
       int32_t col = 0;
       double v = 0.0;
@@ -700,11 +676,11 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
     if (c < ce) {
       nx_cap = a.fcap[c];
       nx_fb = a.fbase[c];
-      if (warp == 7) nx_r0 = a.lrp[c], nx_r1 = a.lrp[c + 1];
+      if (warp == 3) nx_r0 = a.lrp[c], nx_r1 = a.lrp[c + 1];
     }
   };
   facts(cb + 1);
-  unsigned long long gcur = 0, gend = 0;  // the last thread: this block's reserved run of G
+  unsigned long long gcur = 0, gend = 0;  // thread 32: this block's reserved run of G
   // a record whose place is still on its way
   bool pend = false;
   uint32_t p_t = 0, p_s = 0, p_cap = 0, p_x = 0, p_src = 0;
@@ -721,18 +697,18 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
       n = 0;  // skip the column; the host retries with wider buffers
     }
     // ---- sort by (row, source); the last column's records are written -------
-    auto flush = [&] {
-      if (pend) put_record(a, p_t, p_s, p_cap, p_fb, p_x, p_src, p_w);
-      pend = false;
-    };
-    if (n <= RANK_MAX) {
-      const int rank = block_rank(ckey, n, part, flush);
+    if (pend) put_record(a, p_t, p_s, p_cap, p_fb, p_x, p_src, p_w);
+    pend = false;
+    if (n <= EB) {
+      const uint64_t mine = (tid & ((n <= 32 ? 32 : n <= 64 ? 64 : 128) - 1)) < n
+                                ? ckey[tid & ((n <= 32 ? 32 : n <= 64 ? 64 : 128) - 1)]
+                                : 0;
+      const int rank = block_rank(n, part, [&](int f, int) { return (int)(ckey[f] < mine); });
       if (rank >= 0) {
-        bkey[rank] = ckey[tid];
+        bkey[rank] = mine;
         bval[rank] = cval[tid];
       }
     } else {
-      flush();
       if (warp == 0)
         warp_bitonic_sort(ckey, cval, n, [](uint64_t ka, double, uint64_t kb, double) { return ka < kb; });
       __syncthreads();
@@ -746,7 +722,7 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
     const int64_t fb1 = nx_fb, r01 = nx_r0, r11 = nx_r1;
     int32_t row_col = 0;
     double row_v = 0.0;
-    if (more && warp == 7 && r01 + lane < r11) row_col = a.lci[r01 + lane], row_v = a.lv[r01 + lane];
+    if (more && warp == 3 && r01 + lane < r11) row_col = a.lci[r01 + lane], row_v = a.lv[r01 + lane];
     facts(c + 2);
     // ---- duplicates: a row's first record sums the others left to right -----
     int m = 0;
@@ -755,8 +731,7 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
       const int e = e0 + tid;
       int before = m;
 #pragma unroll
-      for (int w = 0; w < EB / 32; ++w) {  // heads of the chunks
-        if (e0 + 32 * w >= n) break;
+      for (int w = 0; w < EB / 32; ++w) {  // heads of the block's four chunks
         const int x = e0 + 32 * w + lane;
         const bool h = x < n && (x == 0 || (uint32_t)(bkey[x - 1] >> 32) != (uint32_t)(bkey[x] >> 32));
         const unsigned bal = __ballot_sync(0xffffffffu, h);
@@ -768,24 +743,7 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
         const uint32_t row = (uint32_t)(bkey[e] >> 32);
         if (e == 0 || (uint32_t)(bkey[e - 1] >> 32) != row) {
           double s = bval[e];
-          for (int f = e + 1; f < n; f += 4) {  // four records read at once
-            uint32_t rw[4];
-            double v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int x = min(f + u, n - 1);
-              rw[u] = f + u < n ? (uint32_t)(bkey[x] >> 32) : ~row;
-              v[u] = bval[x];
-            }
-            if (rw[0] != row) break;
-            s = __dadd_rn(s, v[0]);
-            if (rw[1] != row) break;
-            s = __dadd_rn(s, v[1]);
-            if (rw[2] != row) break;
-            s = __dadd_rn(s, v[2]);
-            if (rw[3] != row) break;
-            s = __dadd_rn(s, v[3]);
-          }
+          for (int f = e + 1; f < n && (uint32_t)(bkey[f] >> 32) == row; ++f) s = __dadd_rn(s, bval[f]);
           akey[before] = row;  // rows ascending
           aval[before] = s;
           wk[before] = wkey(s);
@@ -794,10 +752,16 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
     }
     __syncthreads();
     // ---- sort by (weight, row) ---------------------------------------------
-    if (m <= RANK_MAX) {  // rows ascend, so equal weights order by place
-      const int rank = block_rank(wk, m, part, [] {});
+    if (m <= EB) {
+      const int np = m <= 32 ? 32 : m <= 64 ? 64 : 128, r = tid & (np - 1);
+      const uint64_t mw = r < m ? wk[r] : 0;
+      const uint32_t mr = r < m ? (uint32_t)akey[r] : 0;
+      const int rank = block_rank(m, part, [&](int f, int) {
+        const uint64_t wf = wk[f];
+        return (int)((wf < mw) | ((wf == mw) & ((uint32_t)akey[f] < mr)));
+      });
       if (rank >= 0) {
-        bkey[rank] = (uint32_t)akey[tid];
+        bkey[rank] = mr;
         bval[rank] = aval[tid];
       }
     } else {
@@ -813,54 +777,53 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
     uint4 pre = make_uint4(0u, 0u, 0u, 0u);
     if ((uint32_t)tid < nslab) pre = __ldcg(reinterpret_cast<const uint4 *>(a.frec + fb1 + tid));
     __syncthreads();
-    // ---- prefix sum, uniforms, place in G -----------------------------------
+    // ---- prefix sum (warp 0), uniforms (the others), place in G -------------
     const bool hasg = m > 0 && (int64_t)(uint32_t)akey[m - 1] == ground;
     const int cnt = 1 + m - (hasg ? 1 : 0);
-    double carry = 0.0;
-    for (int e0 = 0; e0 < m; e0 += EB) {  // a chunk of 32 per warp, then the carries in order
-      const int chunks = min(EB / 32, (m - e0 + 31) / 32);
-      double v = 0.0;
-      if (warp < chunks) {
-        const int e = e0 + tid;
-        v = e < m ? bval[e] : 0.0;
+    if (warp == 0) {
+      double carry = 0.0;
+      for (int e0 = 0; e0 < m; e0 += 64) {
+        const int ea = e0 + lane, eb = ea + 32;
+        const bool two = e0 + 32 < m;
+        double va = (ea < m) ? bval[ea] : 0.0, vb = (two && eb < m) ? bval[eb] : 0.0;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-          const double t = __shfl_up_sync(0xffffffffu, v, d);
-          if (lane >= d) v = __dadd_rn(t, v);
-        }
-        if (lane == min(31, m - 1 - e0 - 32 * warp)) s_last[warp] = v;
-      }
-      if (e0 == 0) {
-        for (int i = EB - 1 - tid; i < m - 1; i += EB) uni[i] = uniform53_bits(a.seed, (uint64_t)c, (uint32_t)i);
-        if (tid == EB - 1 && c != ground) {
-          if (gcur + (unsigned)cnt > gend) {
-            const unsigned long long take = max((unsigned)cnt, GCHUNK);
-            gcur = atomicAdd(a.gtop, take);
-            gend = gcur + take;
+          const double ta = __shfl_up_sync(0xffffffffu, va, d);
+          if (lane >= d) va = __dadd_rn(ta, va);
+          if (two) {
+            const double tb = __shfl_up_sync(0xffffffffu, vb, d);
+            if (lane >= d) vb = __dadd_rn(tb, vb);
           }
-          s_gs = gcur;
-          gcur += (unsigned)cnt;
+        }
+        const double outa = __dadd_rn(carry, va);
+        if (ea < m) cs[ea] = outa;
+        carry = __shfl_sync(0xffffffffu, outa, min(31, m - 1 - e0));
+        if (two) {
+          const double outb = __dadd_rn(carry, vb);
+          if (eb < m) cs[eb] = outb;
+          carry = __shfl_sync(0xffffffffu, outb, min(31, m - 1 - e0 - 32));
         }
       }
-      __syncthreads();
-      for (int w = 0; w < chunks; ++w) {
-        if (w == warp) {
-          const double out = __dadd_rn(carry, v);
-          if (e0 + tid < m) cs[e0 + tid] = out;
+    } else {
+      for (int i = tid - 32; i < m - 1; i += EB - 32) uni[i] = uniform53(a.seed, (uint64_t)c, (uint32_t)i);
+      if (tid == 32 && c != ground) {
+        if (gcur + (unsigned)cnt > gend) {
+          const unsigned long long take = max((unsigned)cnt, GCHUNK);
+          gcur = atomicAdd(a.gtop, take);
+          gend = gcur + take;
         }
-        if (w < warp || e0 + EB < m) carry = __dadd_rn(carry, s_last[w]);
+        s_gs = gcur;
+        gcur += (unsigned)cnt;
       }
-      __syncthreads();
     }
+    __syncthreads();
     const double csum = m ? cs[m - 1] : 0.0;
-    // ---- sample: warps 0, 1, 4, 5 search, the others make the weights (edges
-    // up to 64 by warps 0 to 3); warps 4 and 5 the pivot's root and reciprocal;
-    // warp 7 the next column's matrix row ----------------------------------------
-    for (int i0 = (warp & 1) * 32 + (warp >> 2) * 64; i0 < m - 1; i0 += EB / 2) {
+    // ---- sample: even warps search, odd warps make the weights --------------
+    for (int i0 = (warp >> 1) * 32; i0 < m - 1; i0 += EB / 2) {
       const int i = i0 + lane;
       if (i >= m - 1) continue;
       const double tar = cs[i], span = __dsub_rn(csum, tar);
-      if (!(warp & 2)) {
+      if (!(warp & 1)) {
         const uint64_t r = wkey(__dadd_rn(__dmul_rn(uni[i], span), tar));
         int lo = i, hi = m;
         while (lo < hi) {
@@ -873,19 +836,21 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
         wv[i] = __ddiv_rn(__dmul_rn(bval[i], span), csum);
       }
     }
-    if (warp == 4) {
+    if (warp == 2 && c != ground) {
       const double sq = __dsqrt_rn(csum);
       if (lane == 0) {
         s_sq = sq;
         a.diag[c] = csum;
-        if (c != ground && !(csum > 0.0)) atomicOr(&a.flags[FLAG_SINGULAR], 1);
+        if (!(csum > 0.0)) atomicOr(&a.flags[FLAG_SINGULAR], 1);
       }
     }
-    if (warp == 5) {
-      const double inv = __ddiv_rn(1.0, csum);
-      if (lane == 0) s_inv = inv;
-    }
-    if (warp == 7) {
+    if (warp == 3) {
+      if (c != ground) {
+        const double inv = __ddiv_rn(1.0, csum);
+        if (lane == 0) s_inv = inv;
+      } else if (lane == 0) {
+        a.diag[c] = csum;
+      }
       int total = 0;
       if (more) total = put_row(c + 1, r01, r11, row_col, row_v, nkey, nval, (int)nx_all);
       if (lane == 0) s_n[cur ^ 1] = total;
@@ -1097,7 +1062,7 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
           width = std::max(width, initdeg[c] + (int)cap[c]);
       }
       if (nb.empty()) continue;
-      // eight warps per node unless the nodes alone fill the GPU several times
+      // four warps per node unless the nodes alone fill the GPU several times
       const size_t block_bytes = (size_t)std::max(256, pow2_at_least(width)) * 96;
       if ((int64_t)nb.size() <= 8 * (int64_t)prop.multiProcessorCount && block_bytes <= block_limit) {
         keep.emplace_back(nb.size());
