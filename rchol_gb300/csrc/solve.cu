@@ -887,13 +887,28 @@ void pcg_host(const rchol_matrix_s &A, const rchol_factor_s &F, const double *b,
 //
 // The systems are the diagonal blocks of one matrix (rows seg[s] .. seg[s+1])
 // with a block-diagonal factor, so one SpMV and one preconditioner apply serve
-// them all; the scalars of c++/util/pcg.cpp:57-127 are kept per system, one
-// thread block per system computes them (fixed reduction trees, so results
-// are deterministic), and a system stops updating once it has converged.
+// them all; the scalars of c++/util/pcg.cpp:57-127 are kept per system, and a
+// system stops updating once it has converged.  A system's sum is 256 chains
+// over rows 256 apart and a fixed tree over them (so results are
+// deterministic).  Inside the iteration a warp owns 32 of the chains: a system
+// is spread over 8 warps, which may sit on different SMs, each reads 24 rows
+// of its chains ahead, and every kernel that needs a total redoes the tree.  With one
+// thread block per system and a row in flight, 40 systems of 0.85 M rows in all
+// took 170 and 110 us per iteration for the two updates; the sums, updates and
+// stopping test take 77 us now (sums 52: the longest chain's loads).  The order
+// of every sum is the same, which matters: with the
+// factor in FP32, a different rounding here changes iteration counts.
 
 namespace {
 
 constexpr int SEG_THREADS = 256;
+
+unsigned seg_sms() {
+  int dev = 0, sms = 0;
+  RCHOL_CUDA(cudaGetDevice(&dev));
+  RCHOL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  return (unsigned)sms;
+}
 
 struct SegState {
   const int64_t *seg;
@@ -902,6 +917,7 @@ struct SegState {
   int *active, *iters, *any_active;
   const double *tol;
   const int *maxit;
+  double *part;  // [3][nseg][256] chain sums: r.z or p.q, p.r, r.r
 };
 
 // Block-wide sum in a fixed tree; every thread gets the total.
@@ -940,49 +956,118 @@ __global__ void __launch_bounds__(SEG_THREADS) seg_init_kernel(SegState st, cons
   }
 }
 
-// rz = r.z, beta = rz / rz_prev, p = z (first iteration) or beta p + z.
-__global__ void __launch_bounds__(SEG_THREADS) seg_beta_kernel(SegState st, const double *r, const double *z,
-                                                               double *p) {
-  __shared__ double sh[SEG_THREADS];
-  if (!*st.any_active) return;
-  const int s = blockIdx.x;
-  if (!st.active[s]) return;
-  const int64_t i0 = st.seg[s], i1 = st.seg[s + 1];
-  double acc = 0.0;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SEG_THREADS) acc += r[i] * z[i];
-  const double rz = seg_sum(acc, sh);
-  const int it = st.iters[s];
-  const double beta = it == 0 ? 0.0 : rz / st.rz_prev[s];
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SEG_THREADS) p[i] = it == 0 ? z[i] : beta * p[i] + 1.0 * z[i];
-  if (threadIdx.x == 0) st.rz[s] = rz;
+constexpr int SEG_GROUPS = SEG_THREADS / 32;  // warps of a system
+constexpr int SEG_AHEAD = 24;                 // rows of a chain read at a time
+
+// This warp's system (-1: none left, or converged) and chains.
+struct SegLane {
+  int s, chain;
+  int64_t i0, i1;
+};
+__device__ __forceinline__ SegLane seg_lane(const SegState &st) {
+  SegLane g{-1, 0, 0, 0};
+  const int w = (int)(blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32), s = w / SEG_GROUPS;
+  if (s >= st.nseg || !*st.any_active || !st.active[s]) return g;
+  g.s = s;
+  g.chain = (w % SEG_GROUPS) * 32 + (int)(threadIdx.x & 31);
+  g.i0 = st.seg[s] + g.chain;
+  g.i1 = st.seg[s + 1];
+  return g;
 }
 
-// alpha = p.r / p.q, x += alpha p, r -= alpha q, then the stopping test.
+// The tree of seg_sum over a system's 256 chain sums, by one warp: lane l holds
+// chains l + 32 m.  Every lane gets the total.
+__device__ __forceinline__ double seg_total(const double *chains) {
+  const int lane = threadIdx.x & 31;
+  double v[SEG_GROUPS];
+#pragma unroll
+  for (int m = 0; m < SEG_GROUPS; ++m) v[m] = chains[lane + 32 * m];
+#pragma unroll
+  for (int h = SEG_GROUPS / 2; h > 0; h >>= 1)
+#pragma unroll
+    for (int m = 0; m < h; ++m) v[m] += v[m + h];
+#pragma unroll
+  for (int h = 16; h > 0; h >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], h);
+  return v[0];
+}
+
+__device__ __forceinline__ double *seg_chains(const SegState &st, int which, int s) {
+  return st.part + ((size_t)which * st.nseg + s) * SEG_THREADS;
+}
+
+// Chain sums of a.b, and of a.c where c is given (DUAL).
+template <bool DUAL>
+__global__ void __launch_bounds__(32) seg_dot_kernel(SegState st, int which, const double *__restrict__ a,
+                                                     const double *__restrict__ b, const double *__restrict__ c) {
+  const SegLane g = seg_lane(st);
+  if (g.s < 0) return;
+  double s0 = 0.0, s1 = 0.0;
+  for (int64_t i = g.i0; i < g.i1; i += SEG_AHEAD * SEG_THREADS) {
+    double av[SEG_AHEAD], bv[SEG_AHEAD], cv[SEG_AHEAD];
+#pragma unroll
+    for (int u = 0; u < SEG_AHEAD; ++u) {
+      const int64_t k = i + u * SEG_THREADS;
+      const bool on = k < g.i1;
+      av[u] = on ? a[k] : 0.0;
+      bv[u] = on ? b[k] : 0.0;
+      if (DUAL) cv[u] = on ? c[k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < SEG_AHEAD; ++u)
+      if (i + u * SEG_THREADS < g.i1) {
+        s0 += av[u] * bv[u];
+        if (DUAL) s1 += av[u] * cv[u];
+      }
+  }
+  seg_chains(st, which, g.s)[g.chain] = s0;
+  if (DUAL) seg_chains(st, which + 1, g.s)[g.chain] = s1;
+}
+
+// beta = rz / rz_prev, p = z (first iteration) or beta p + z; grid (systems, parts).
+__global__ void __launch_bounds__(SEG_THREADS) seg_beta_kernel(SegState st, const double *z, double *p) {
+  __shared__ double sh;
+  const int s = blockIdx.x;
+  if (!*st.any_active || !st.active[s]) return;
+  if (threadIdx.x < 32) {
+    const double rz = seg_total(seg_chains(st, 0, s));
+    if (threadIdx.x == 0) sh = rz;
+  }
+  __syncthreads();
+  const double rz = sh;
+  const int it = st.iters[s];
+  const double beta = it == 0 ? 0.0 : rz / st.rz_prev[s];
+  const int64_t i1 = st.seg[s + 1];
+  for (int64_t i = st.seg[s] + blockIdx.y * SEG_THREADS + threadIdx.x; i < i1; i += (int64_t)gridDim.y * SEG_THREADS)
+    p[i] = it == 0 ? z[i] : beta * p[i] + 1.0 * z[i];
+  if (threadIdx.x == 0 && blockIdx.y == 0) st.rz[s] = rz;
+}
+
+// alpha = p.r / p.q, x += alpha p, r -= alpha q; grid (systems, parts).
 __global__ void __launch_bounds__(SEG_THREADS) seg_alpha_kernel(SegState st, const double *p, const double *q,
                                                                 double *x, double *r) {
-  __shared__ double sh[SEG_THREADS];
-  if (!*st.any_active) return;
+  __shared__ double sh;
   const int s = blockIdx.x;
-  if (!st.active[s]) return;
-  const int64_t i0 = st.seg[s], i1 = st.seg[s + 1];
-  double a0 = 0.0, a1 = 0.0;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SEG_THREADS) {
-    const double pv = p[i];
-    a0 += pv * q[i];
-    a1 += pv * r[i];
+  if (!*st.any_active || !st.active[s]) return;
+  if (threadIdx.x < 32) {
+    const double pq = seg_total(seg_chains(st, 0, s)), pr = seg_total(seg_chains(st, 1, s));
+    if (threadIdx.x == 0) sh = pr / pq;
   }
-  const double pq = seg_sum(a0, sh);
-  const double pr = seg_sum(a1, sh);
-  const double alpha = pr / pq;
-  double rr = 0.0;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SEG_THREADS) {
+  __syncthreads();
+  const double alpha = sh;
+  const int64_t i1 = st.seg[s + 1];
+  for (int64_t i = st.seg[s] + blockIdx.y * SEG_THREADS + threadIdx.x; i < i1;
+       i += (int64_t)gridDim.y * SEG_THREADS) {
     x[i] += alpha * p[i];
-    const double rv = r[i] + -alpha * q[i];
-    r[i] = rv;
-    rr += rv * rv;
+    r[i] = r[i] + -alpha * q[i];
   }
-  const double t = seg_sum(rr, sh);
-  if (threadIdx.x == 0) {
+}
+
+// The stopping test, one warp per system.
+__global__ void __launch_bounds__(128) seg_conv_kernel(SegState st) {
+  const int s = (int)(blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32);
+  if (s >= st.nseg || !*st.any_active || !st.active[s]) return;
+  const double t = seg_total(seg_chains(st, 2, s));
+  if ((threadIdx.x & 31) == 0) {
     const int it = st.iters[s] + 1;
     st.iters[s] = it;
     st.rz_prev[s] = st.rz[s];
@@ -1035,7 +1120,7 @@ static SegWork &seg_workspace(const rchol_matrix_s &A, const rchol_factor_s &F, 
   w->p.alloc(A.n);
   w->q.alloc(A.n);
   w->x.alloc(A.n);
-  w->sc.alloc(4 * (size_t)nseg + 1);
+  w->sc.alloc(4 * (size_t)nseg + 1 + 3 * (size_t)nseg * SEG_THREADS);
   w->ic.alloc(2 * (size_t)nseg + 2);
   RCHOL_CUDA(cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking));
   RCHOL_CUDA(cudaEventCreateWithFlags(&w->ev_in, cudaEventDisableTiming));
@@ -1059,6 +1144,7 @@ static SegState seg_state(SegWork &w) {
   st.iters = w.ic.p + S;
   st.any_active = w.ic.p + 2 * (size_t)S;
   st.maxit = w.ic.p + 2 * (size_t)S + 1;
+  st.part = w.sc.p + 4 * (size_t)S + 1;
   return st;
 }
 
@@ -1089,9 +1175,16 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
     RCHOL_CUDA(cudaStreamBeginCapture(ws, cudaStreamCaptureModeThreadLocal));
     try {
       precond_ready(F, pcg_blocks(F), w.r.p, w.z.p, 1, ws);
-      seg_beta_kernel<<<S, SEG_THREADS, 0, ws>>>(st, w.r.p, w.z.p, w.p.p);
+      const unsigned C = S * SEG_GROUPS;
+      // element updates: enough parts of a system for four thread blocks an SM
+      const dim3 E(S, std::min(64u, (4 * seg_sms() + S - 1) / S));
+      seg_dot_kernel<false><<<C, 32, 0, ws>>>(st, 0, w.r.p, w.z.p, nullptr);
+      seg_beta_kernel<<<E, SEG_THREADS, 0, ws>>>(st, w.z.p, w.p.p);
       spmv(A, w.p.p, w.q.p, 1, ws);
-      seg_alpha_kernel<<<S, SEG_THREADS, 0, ws>>>(st, w.p.p, w.q.p, w.x.p, w.r.p);
+      seg_dot_kernel<true><<<C, 32, 0, ws>>>(st, 0, w.p.p, w.q.p, w.r.p);
+      seg_alpha_kernel<<<E, SEG_THREADS, 0, ws>>>(st, w.p.p, w.q.p, w.x.p, w.r.p);
+      seg_dot_kernel<false><<<C, 32, 0, ws>>>(st, 2, w.r.p, w.r.p, nullptr);
+      seg_conv_kernel<<<(S + 3) / 4, 128, 0, ws>>>(st);
       seg_any_kernel<<<1, 256, 0, ws>>>(st);
       RCHOL_CUDA(cudaGetLastError());
     } catch (...) {
