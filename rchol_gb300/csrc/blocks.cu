@@ -14,6 +14,12 @@
 // memory; t and x travel as remote stores that complete on the receivers'
 // mbarriers, so a step has two one-way trips and no cluster barrier.
 //
+// Several right-hand sides lie column after column, and a cluster solves one
+// column of a piece: the chain's length, not the arithmetic, is what a solve
+// costs, and columns hide it from one another.  Preconditioner of 80^3 with
+// 128 subdomains, record streams -> now: FP32 2 columns 8.9 -> 0.65 ms, 32
+// columns 8.3 -> 2.6; FP64 49 -> 1.5 and 49 -> 8.8 ms.
+//
 // The plan is built on the GPU from the CSR of G (or G^T): count entries by
 // distance, lay out the records, copy the entries, invert the triangles.
 
@@ -351,17 +357,22 @@ __global__ void __launch_bounds__(32) blk_invert_kernel(const BlkRec *recs, BlkI
 // ---- solving ----------------------------------------------------------------------------------
 
 // acc_i = in_i - (entries of row i in a CSR of external ones) out, LANES
-// lanes per row, four entries in flight per lane; in may be acc.
-template <typename VT, typename InT, typename OutT, int LANES>
+// lanes per row, four entries in flight per lane; in may be acc.  One
+// right-hand side (KC = 1), or columns (n apart) KC blockIdx.y and on of k, so
+// that a row's entries are read once for KC of them.
+template <typename VT, typename InT, typename OutT, int LANES, int KC>
 __global__ void __launch_bounds__(256) blk_ext_kernel(const int32_t *__restrict__ rows, int64_t nrows,
                                                         const int64_t *__restrict__ rp, const int32_t *__restrict__ ci,
                                                         const VT *__restrict__ v, const InT *in,
-                                                        const OutT *__restrict__ out, VT *acc) {
+                                                        const OutT *__restrict__ out, VT *acc, int k, int64_t n) {
   const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LANES;
-  const int sub = threadIdx.x % LANES;
+  const int sub = threadIdx.x % LANES, col0 = KC == 1 ? 0 : blockIdx.y * KC;
   if (t >= nrows) return;  // whole groups leave together
   const int64_t i = rows[t], q1 = rp[i + 1];
-  VT s[4] = {VT(0), VT(0), VT(0), VT(0)};
+  const OutT *oc[KC];
+#pragma unroll
+  for (int j = 0; j < KC; ++j) oc[j] = KC == 1 ? out : out + min(col0 + j, k - 1) * n;
+  VT s[KC][4] = {};
   for (int64_t q = rp[i] + sub; q < q1; q += 4 * LANES) {
     int32_t c[4];
     VT w[4];
@@ -373,13 +384,20 @@ __global__ void __launch_bounds__(256) blk_ext_kernel(const int32_t *__restrict_
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (c[u] >= 0) s[u] = fma(w[u], (VT)out[c[u]], s[u]);
+      if (c[u] >= 0) {
+#pragma unroll
+        for (int j = 0; j < KC; ++j) s[j][u] = fma(w[u], (VT)oc[j][c[u]], s[j][u]);
+      }
   }
-  VT sum = (s[0] + s[1]) + (s[2] + s[3]);
   const unsigned mask = LANES == 32 ? 0xffffffffu : (((1u << LANES) - 1u) << ((threadIdx.x & 31) / LANES * LANES));
 #pragma unroll
-  for (int o = LANES / 2; o; o >>= 1) sum += __shfl_xor_sync(mask, sum, o, LANES);
-  if (sub == 0) acc[i] = (VT)in[i] - sum;
+  for (int j = 0; j < KC; ++j) {
+    VT sum = (s[j][0] + s[j][1]) + (s[j][2] + s[j][3]);
+#pragma unroll
+    for (int o = LANES / 2; o; o >>= 1) sum += __shfl_xor_sync(mask, sum, o, LANES);
+    const int64_t at = KC == 1 ? i : (col0 + j) * n + i;
+    if (sub == 0 && (KC == 1 || col0 + j < k)) acc[at] = (VT)in[at] - sum;
+  }
 }
 
 template <typename VT>
@@ -395,6 +413,8 @@ struct BlkArgs {
   int ring, slot;
   int fused;  // the records hold external entries
   int xrows;  // positions of the unknowns' array (four zeros follow)
+  int k;      // right-hand sides, columns n apart
+  int64_t n;
   int32_t goff[kBlkMaxGroups + 1];
 };
 
@@ -549,7 +569,16 @@ __global__ void __launch_bounds__(512) blk_solve_kernel(BlkArgs<VT> a, const InT
   extern __shared__ __align__(16) unsigned char smem[];
   const int C = CLUSTER ? a.C : 1;
   const int rank = CLUSTER ? (int)(blockIdx.x % (unsigned)C) : 0;
-  const BlkPiece pc = a.pieces[CLUSTER ? blockIdx.x / (unsigned)C : blockIdx.x];
+  // a cluster takes one column of a piece; the columns of a piece run side by
+  // side, so its records and inverses come from L2 for all but one of them
+  unsigned item = CLUSTER ? blockIdx.x / (unsigned)C : blockIdx.x;
+  if (a.k > 1) {
+    const int64_t col = item % (unsigned)a.k;
+    item /= (unsigned)a.k;
+    in += col * a.n;
+    out += col * a.n;
+  }
+  const BlkPiece pc = a.pieces[item];
   const int tid = threadIdx.x, T = blockDim.x, B = a.B, nb = pc.nblocks, rows = pc.rows;
   const int nown = B / C, GL = a.gl, LD = GL >> 2, TC = nown * LD;
   constexpr int per = 16 / (int)sizeof(VT);
@@ -834,8 +863,8 @@ namespace {
 // In FP64 (2 FMA per clock and SM) the inverse's B / 2 products per row are
 // what a step costs, so B is smaller: 417 us for 64^3 with 64 subdomains
 // against 451 with B = 128 at the root and 1066 with the record streams.
-void choose_shape(BlkStage &S, bool fp32) {
-  const int P = S.npieces, R = S.maxrows;
+void choose_shape(BlkStage &S, bool fp32, int cols) {
+  const int P = (int)std::min<int64_t>((int64_t)S.npieces * cols, 1 << 20), R = S.maxrows;
   const int i = P <= 8 && R >= 512 ? 4 : P <= 18 && R >= 256 ? 3 : P <= 36 && R >= 128 ? 2 : P <= 76 && R >= 128 ? 1 : 0;
   static const int b32[] = {64, 128, 256, 256, 512}, b64[] = {32, 64, 128, 128, 256};
   static const int g32[] = {8, 16, 16, 32, 32}, g64[] = {16, 16, 32, 32, 32};
@@ -872,7 +901,7 @@ size_t stage_smem(const BlkStage &S, size_t vsz, int ring) {
 
 template <typename VT>
 bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, const DevBuf<double> &v,
-               const std::vector<TreeNode> &tnodes, bool upper, BlkDir &D, DevBuf<VT> &inv, cudaStream_t s) {
+               const std::vector<TreeNode> &tnodes, bool upper, int cols, BlkDir &D, DevBuf<VT> &inv, cudaStream_t s) {
   int maxdepth = 1;
   for (auto &nd : tnodes) maxdepth = std::max(maxdepth, nd.depth);
   std::vector<BlkPiece> pieces;
@@ -899,7 +928,7 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
       }
       S.npieces = (int)pieces.size() - S.piece0;
       if (!S.npieces) break;
-      choose_shape(S, sizeof(VT) == 4);
+      choose_shape(S, sizeof(VT) == 4, cols);
       D.stages.push_back(S);
     }
   }
@@ -1069,10 +1098,10 @@ void launch_stage(const BlkStage &S, const BlkArgs<VT> &a, const InT *in, OutT *
   });
   const unsigned threads = (unsigned)(S.B / S.C / 4 * S.gl + S.helpers);
   if (S.C == 1) {
-    single<<<S.npieces, threads, S.smem, s>>>(a, in, out);
+    single<<<(unsigned)S.npieces * (unsigned)a.k, threads, S.smem, s>>>(a, in, out);
   } else {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(S.npieces * S.C));
+    cfg.gridDim = dim3((unsigned)S.npieces * (unsigned)a.k * (unsigned)S.C);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = S.smem;
     cfg.stream = s;
@@ -1106,26 +1135,33 @@ const double *ext_values<double>(const BlkExt &E) {
   return E.v64.p;
 }
 
-template <typename VT, typename InT, typename OutT>
-void launch_ext(const BlkExt &E, int lanes, const int32_t *rows, int64_t nrows, const InT *in, const OutT *out, VT *acc,
-                cudaStream_t s) {
-  const unsigned grid = (unsigned)((nrows * lanes + 255) / 256);
+template <typename VT, typename InT, typename OutT, int KC>
+void launch_ext_kc(const BlkExt &E, int lanes, const int32_t *rows, int64_t nrows, const InT *in, const OutT *out,
+                   VT *acc, int k, int64_t n, cudaStream_t s) {
+  const dim3 grid((unsigned)((nrows * lanes + 255) / 256), (unsigned)((k + KC - 1) / KC));
   const VT *v = ext_values<VT>(E);
-  if (lanes == 2) blk_ext_kernel<VT, InT, OutT, 2><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc);
-  else if (lanes == 8) blk_ext_kernel<VT, InT, OutT, 8><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc);
-  else blk_ext_kernel<VT, InT, OutT, 32><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc);
+  if (lanes == 2) blk_ext_kernel<VT, InT, OutT, 2, KC><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
+  else if (lanes == 8) blk_ext_kernel<VT, InT, OutT, 8, KC><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
+  else blk_ext_kernel<VT, InT, OutT, 32, KC><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
   note_launch();
   RCHOL_CUDA(cudaGetLastError());
 }
 
+template <typename VT, typename InT, typename OutT>
+void launch_ext(const BlkExt &E, int lanes, const int32_t *rows, int64_t nrows, const InT *in, const OutT *out, VT *acc,
+                int k, int64_t n, cudaStream_t s) {
+  if (k == 1) launch_ext_kc<VT, InT, OutT, 1>(E, lanes, rows, nrows, in, out, acc, k, n, s);
+  else launch_ext_kc<VT, InT, OutT, 4>(E, lanes, rows, nrows, in, out, acc, k, n, s);
+}
+
 template <typename VT, typename InT, typename OutT, bool UPPER>
-void launch_dir(const BlkDir &D, const VT *inv, const InT *in, OutT *out, VT *acc, unsigned int *status,
-                cudaStream_t s) {
+void launch_dir(const BlkDir &D, const VT *inv, const InT *in, OutT *out, VT *acc, int k, int64_t n,
+                unsigned int *status, cudaStream_t s) {
   for (size_t st = 0; st < D.stages.size(); ++st) {
     const BlkStage &S = D.stages[st];
     if (st == 1 && D.early_rows)
-      launch_ext<VT, InT, OutT>(D.early, D.early.lanes, D.erow.p, D.early_rows, in, out, acc, s);
-    if (S.late_lanes) launch_ext<VT, VT, OutT>(D.late, S.late_lanes, D.erow.p + S.erow0, S.rows, acc, out, acc, s);
+      launch_ext<VT, InT, OutT>(D.early, D.early.lanes, D.erow.p, D.early_rows, in, out, acc, k, n, s);
+    if (S.late_lanes) launch_ext<VT, VT, OutT>(D.late, S.late_lanes, D.erow.p + S.erow0, S.rows, acc, out, acc, k, n, s);
     BlkArgs<VT> a;
     a.pieces = D.pieces.p + S.piece0;
     a.rec_off = D.rec_off.p;
@@ -1141,16 +1177,25 @@ void launch_dir(const BlkDir &D, const VT *inv, const InT *in, OutT *out, VT *ac
     a.slot = S.slot;
     a.fused = S.fused;
     a.xrows = (S.maxrows + 3) / 4 * 4;
+    a.k = k;
+    a.n = n;
     std::copy(S.goff, S.goff + kBlkMaxGroups + 1, a.goff);
     if (st > 0 && D.early_rows) launch_nv<VT, VT, OutT, UPPER>(S, a, acc, out, s);
     else launch_nv<VT, InT, OutT, UPPER>(S, a, in, out, s);
   }
 }
 
+bool build_block_dirs(const rchol_factor_s &F, int cols, BlkDir &fwd, BlkDir &bwd, cudaStream_t s) {
+  if (F.precision == RCHOL_PREC_FP32)
+    return build_dir<float>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv32, s) &&
+           build_dir<float>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv32, s);
+  return build_dir<double>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv64, s) &&
+         build_dir<double>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv64, s);
+}
+
 }  // namespace
 
 bool build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
-  const bool fp32 = F.precision == RCHOL_PREC_FP32;
   // Inverses of large triangles are as accurate as substitution because
   // nothing cancels in them: the diagonal is positive and no other entry is
   // (true of every sampled factor).  Any other G keeps the record streams.
@@ -1162,31 +1207,34 @@ bool build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
   positive.download(count, 2, s);
   RCHOL_CUDA(cudaStreamSynchronize(s));
   if (count[0] != (unsigned long long)F.n || count[1] != (unsigned long long)F.n) return false;
-  return fp32 ? build_dir<float>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, P.bfwd, P.bfwd.inv32, s) &&
-                    build_dir<float>(F.n, F.urp, F.uci, F.uv, F.nodes, true, P.bbwd, P.bbwd.inv32, s)
-              : build_dir<double>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, P.bfwd, P.bfwd.inv64, s) &&
-                    build_dir<double>(F.n, F.urp, F.uci, F.uv, F.nodes, true, P.bbwd, P.bbwd.inv64, s);
+  return build_block_dirs(F, 1, P.bfwd, P.bbwd, s);
+}
+
+void build_blocks_k(const rchol_factor_s &F, SolvePlan &P, int k, cudaStream_t s) {
+  if (P.kblocks || k < kBlkWideFrom) return;
+  P.kwide = build_block_dirs(F, kBlkWideCols, P.bkfwd, P.bkbwd, s);
+  P.kblocks = true;
 }
 
 void block_trsv(const rchol_factor_s &F, const SolvePlan &P, bool upper, const double *in64, const float *in32,
-                double *out64, float *out32, void *acc, cudaStream_t s) {
+                double *out64, float *out32, void *acc, int k, cudaStream_t s) {
   unsigned int *st = P.status;
   float *a32 = static_cast<float *>(acc);
   double *a64 = static_cast<double *>(acc);
+  const int64_t n = F.n;
+  const bool wide = P.kwide && k >= kBlkWideFrom;
+  const BlkDir &D = upper ? wide ? P.bkbwd : P.bbwd : wide ? P.bkfwd : P.bfwd;
   if (F.precision == RCHOL_PREC_FP32) {
-    if (!upper && in64 && out32)
-      launch_dir<float, double, float, false>(P.bfwd, P.bfwd.inv32.p, in64, out32, a32, st, s);
-    else if (!upper && in64 && out64)
-      launch_dir<float, double, double, false>(P.bfwd, P.bfwd.inv32.p, in64, out64, a32, st, s);
-    else if (upper && in32 && out64)
-      launch_dir<float, float, double, true>(P.bbwd, P.bbwd.inv32.p, in32, out64, a32, st, s);
-    else if (upper && in64 && out64)
-      launch_dir<float, double, double, true>(P.bbwd, P.bbwd.inv32.p, in64, out64, a32, st, s);
+    const float *inv = D.inv32.p;
+    if (!upper && in64 && out32) launch_dir<float, double, float, false>(D, inv, in64, out32, a32, k, n, st, s);
+    else if (!upper && in64 && out64) launch_dir<float, double, double, false>(D, inv, in64, out64, a32, k, n, st, s);
+    else if (upper && in32 && out64) launch_dir<float, float, double, true>(D, inv, in32, out64, a32, k, n, st, s);
+    else if (upper && in64 && out64) launch_dir<float, double, double, true>(D, inv, in64, out64, a32, k, n, st, s);
     else throw Error(RCHOL_ERR_INTERNAL, "unsupported triangular-solve operand types");
   } else {
     if (!in64 || !out64) throw Error(RCHOL_ERR_INTERNAL, "unsupported triangular-solve operand types");
-    if (upper) launch_dir<double, double, double, true>(P.bbwd, P.bbwd.inv64.p, in64, out64, a64, st, s);
-    else launch_dir<double, double, double, false>(P.bfwd, P.bfwd.inv64.p, in64, out64, a64, st, s);
+    if (upper) launch_dir<double, double, double, true>(D, D.inv64.p, in64, out64, a64, k, n, st, s);
+    else launch_dir<double, double, double, false>(D, D.inv64.p, in64, out64, a64, k, n, st, s);
   }
 }
 

@@ -76,6 +76,15 @@ struct StreamDir {
 
 constexpr int kBlkMaxRows = 16384;  // a piece's unknowns in shared memory: 64 KB in FP32, 128 KB in FP64
 constexpr int kBlkMaxGroups = 64;   // 4-row groups of a thread block
+constexpr int kBlkCols = 32;        // right-hand sides of one traversal
+// From kBlkWideFrom right-hand sides on, the solves run on a second plan whose
+// shapes count every piece kBlkWideCols times: the columns fill the GPU, so
+// clusters are smaller and blocks shorter.  us per preconditioner, first plan /
+// second, FP32: 80^3 2 columns 651 / 693, 5 columns 926 / 784, 32 columns
+// 4020 / 2605; 30^3 2 columns 134 / 164, 5 columns 192 / 168; FP64 80^3 2
+// columns 1483 / 1622, 5 columns 2348 / 2139.  With pieces counted 4 times
+// 32 columns take 2900 us, 32 times 2448 (but 5 columns 998).
+constexpr int kBlkWideFrom = 5, kBlkWideCols = 8;
 
 struct BlkPiece {
   int64_t begin;   // first row
@@ -189,6 +198,8 @@ struct SolvePlan {
   unsigned int *status = nullptr;  // status word of the solve kernels
   bool blocked = false;    // the solves run on bfwd / bbwd (else, and in an FP32 PCG, on the record streams)
   BlkDir bfwd, bbwd;
+  BlkDir bkfwd, bkbwd;     // shapes for several right-hand sides (built on first use)
+  bool kblocks = false, kwide = false;  // that was tried; it is there
   StreamDir sfwd, sbwd;
   StreamDir kfwd, kbwd;    // pieces for up to 32 right-hand sides (built on first use)
   bool kbuilt = false;
@@ -199,14 +210,17 @@ struct SolvePlan {
   DevBuf<float> acc32;
   DevBuf<double> acck64;   // the same for up to 32 right-hand sides (n x 32)
   DevBuf<float> acck32;
+  DevBuf<double> colk;     // right-hand sides and solutions column after column
 };
 
 // Block plan of both directions; false if G's rows are too dense for it.
 bool build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
-// Solve with G (upper = false) or G^T for one right-hand side; acc: n values
-// of G's precision.
+// The plan that k right-hand sides take, where it is another one.
+void build_blocks_k(const rchol_factor_s &F, SolvePlan &P, int k, cudaStream_t s);
+// Solve with G (upper = false) or G^T for k <= kBlkCols right-hand sides, one
+// column after another; acc: n k values of G's precision.
 void block_trsv(const rchol_factor_s &F, const SolvePlan &P, bool upper, const double *in64, const float *in32,
-                double *out64, float *out32, void *acc, cudaStream_t s);
+                double *out64, float *out32, void *acc, int k, cudaStream_t s);
 // Device address of the status word of the solve kernels (current device).
 unsigned int *solve_status_word();
 void build_streams(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);

@@ -500,7 +500,7 @@ static void ensure_scratch(SolvePlan &P, bool fp32, int64_t count) {
 // values of G's precision.
 static void trsv_one(const rchol_factor_s &F, const SolvePlan &P, bool blocks, bool upper, const double *in64,
                      const float *in32, double *out64, float *out32, void *acc, cudaStream_t s) {
-  if (blocks) block_trsv(F, P, upper, in64, in32, out64, out32, acc, s);
+  if (blocks) block_trsv(F, P, upper, in64, in32, out64, out32, acc, 1, s);
   else stream_trsv(F, P, upper, in64, in32, out64, out32, acc, s);
 }
 
@@ -521,6 +521,84 @@ static void *ensure_acc(SolvePlan &P, bool fp32, int64_t n) {
   return P.acc64.p;
 }
 
+// What k right-hand sides need beyond ensure_scratch, on the block plan or the
+// record streams.
+static void ensure_k(const rchol_factor_s &F, bool blocks, int k, cudaStream_t s) {
+  SolvePlan &P = *F.plan;
+  const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  if (k == 1) {
+    ensure_acc(P, fp32, F.n);
+    return;
+  }
+  if (!blocks) {
+    build_streams_k(F, P, s);
+    return;
+  }
+  build_blocks_k(F, P, std::min(k, kBlkCols), s);
+  const size_t all = (size_t)F.n * kBlkCols, cols = 2 * (size_t)F.n * std::min(k, kBlkCols);
+  if (fp32 && P.acck32.n < all) P.acck32.alloc(all);
+  if (!fp32 && P.acck64.n < all) P.acck64.alloc(all);
+  if (P.colk.n < cols) {
+    P.colk.alloc(cols);
+    P.pcg.clear();  // their graphs hold the old address
+    P.seg.clear();
+  }
+}
+
+// Columns j0 .. j0 + g of an n x k row-major array, one after another
+// (TO_COLS), or back.  A thread block moves 64 rows through shared memory, so
+// both sides are read and written in runs.
+template <bool TO_COLS>
+__global__ void __launch_bounds__(256) blk_columns_kernel(int64_t n, int k, int j0, int g, const double *__restrict__ in,
+                                                          double *__restrict__ out) {
+  __shared__ double tile[64][kBlkCols + 1];
+  const int64_t r0 = blockIdx.x * (int64_t)64;
+  const int rows = (int)min((int64_t)64, n - r0);
+  for (int e = threadIdx.x; e < 64 * g; e += 256) {
+    const int r = TO_COLS ? e / g : e & 63, c = TO_COLS ? e - r * g : e >> 6;
+    if (r < rows) tile[r][c] = TO_COLS ? in[(r0 + r) * k + j0 + c] : in[c * n + r0 + r];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 64 * g; e += 256) {
+    const int r = TO_COLS ? e & 63 : e / g, c = TO_COLS ? e >> 6 : e - r * g;
+    if (r >= rows) continue;
+    if (TO_COLS) out[c * n + r0 + r] = tile[r][c];
+    else out[(r0 + r) * k + j0 + c] = tile[r][c];
+  }
+}
+
+template <bool TO_COLS>
+static void move_columns(int64_t n, int k, int j0, int g, const double *in, double *out, cudaStream_t s) {
+  blk_columns_kernel<TO_COLS><<<(unsigned)((n + 63) / 64), 256, 0, s>>>(n, k, j0, g, in, out);
+  note_launch();
+  RCHOL_CUDA(cudaGetLastError());
+}
+
+// k right-hand sides (n x k row-major) on the block plan, up to kBlkCols
+// columns at a time: the solve of direction `dir` (0, 1) or the preconditioner (2).
+static void blocks_k(const rchol_factor_s &F, const SolvePlan &P, int dir, const double *in, double *out, int k,
+                     cudaStream_t s) {
+  const int64_t n = F.n;
+  const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  void *acc = fp32 ? (void *)P.acck32.p : (void *)P.acck64.p;
+  double *a = P.colk.p;
+  for (int j0 = 0; j0 < k; j0 += kBlkCols) {
+    const int g = std::min(kBlkCols, k - j0);
+    double *b = a + n * g;
+    move_columns<true>(n, k, j0, g, in, a, s);
+    if (dir < 2) {
+      block_trsv(F, P, dir == 1, a, nullptr, b, nullptr, acc, g, s);
+    } else if (fp32) {
+      block_trsv(F, P, false, a, nullptr, nullptr, P.ytmp32.p, acc, g, s);
+      block_trsv(F, P, true, nullptr, P.ytmp32.p, b, nullptr, acc, g, s);
+    } else {
+      block_trsv(F, P, false, a, nullptr, P.ytmp.p, nullptr, acc, g, s);
+      block_trsv(F, P, true, P.ytmp.p, nullptr, b, nullptr, acc, g, s);
+    }
+    move_columns<false>(n, k, j0, g, b, out, s);
+  }
+}
+
 // The preconditioner with the plan's buffers already sized (inside PCG).
 static void precond_ready(const rchol_factor_s &F, bool blocks, const double *r, double *z, int k, cudaStream_t s);
 
@@ -529,19 +607,17 @@ void trsv(const rchol_factor_s &F, bool upper, const double *in, double *out, in
   std::lock_guard<std::mutex> guard(P.lock);
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   ensure_scratch(P, fp32, F.n * k);
-  if (k == 1) {
-    trsv_one(F, P, P.blocked, upper, in, nullptr, out, nullptr, ensure_acc(P, fp32, F.n), s);
-    return;
-  }
-  build_streams_k(F, P, s);
-  stream_trsv_k(F, P, upper, in, nullptr, out, nullptr, k, s);
+  ensure_k(F, P.blocked, k, s);
+  if (k == 1) trsv_one(F, P, P.blocked, upper, in, nullptr, out, nullptr, ensure_acc(P, fp32, F.n), s);
+  else if (P.blocked) blocks_k(F, P, upper, in, out, k, s);
+  else stream_trsv_k(F, P, upper, in, nullptr, out, nullptr, k, s);
 }
 
 void precond(const rchol_factor_s &F, const double *r, double *z, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
   ensure_scratch(P, F.precision == RCHOL_PREC_FP32, F.n * k);
-  if (k > 1) build_streams_k(F, P, s);
+  ensure_k(F, P.blocked, k, s);
   precond_ready(F, P.blocked, r, z, k, s);
 }
 
@@ -553,9 +629,9 @@ static void precond_ready(const rchol_factor_s &F, bool blocks, const double *r,
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   if (k == 1) {
     precond_one(F, P, blocks, r, z, P.ytmp.p, P.ytmp32.p, ensure_acc(P, fp32, F.n), s);
-    return;
-  }
-  if (fp32) {
+  } else if (blocks) {
+    blocks_k(F, P, 2, r, z, k, s);
+  } else if (fp32) {
     stream_trsv_k(F, P, false, r, nullptr, nullptr, P.ytmp32.p, k, s);
     stream_trsv_k(F, P, true, nullptr, P.ytmp32.p, z, nullptr, k, s);
   } else {
@@ -800,8 +876,7 @@ static void pcg_impl(const rchol_matrix_s &A, const rchol_factor_s &F, const dou
   const int64_t n = A.n, nk = n * k;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   ensure_scratch(P, fp32, nk);
-  if (k > 1) build_streams_k(F, P, s);
-  ensure_acc(P, fp32, n);
+  ensure_k(F, pcg_blocks(F), k, s);
   PcgWork &w = pcg_workspace(A, F, k);
   PcgState st = pcg_state(w);
   cudaStream_t ws = w.stream;

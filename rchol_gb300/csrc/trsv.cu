@@ -1,7 +1,7 @@
 // Block triangular solves with G (forward) and G^T (backward) from streams of
-// 32-row records: several right-hand sides at once, factors whose rows are too
-// dense for the large blocks of blocks.cu or whose entries have mixed signs,
-// and the formats that RCHOL_TRSV_FORMAT names.
+// 32-row records: PCG with G in FP32, factors whose rows are too dense for the
+// large blocks of blocks.cu or whose entries have mixed signs, and the formats
+// that RCHOL_TRSV_FORMAT names.
 //
 // Replaces the two MKL trsv calls of c++/util/pcg.cpp:141-159.
 //
@@ -2063,8 +2063,11 @@ void build_streams(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
 void build_streams_k(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
   if (P.kbuilt) return;
   build_streams_width(F, KW, P.kfwd, P.kbwd, s);
-  if (F.precision == RCHOL_PREC_FP32) P.acck32.alloc((size_t)F.n * KW);
-  else P.acck64.alloc((size_t)F.n * KW);
+  const size_t nacc = (size_t)F.n * KW;
+  if (F.precision == RCHOL_PREC_FP32 ? P.acck32.n < nacc : P.acck64.n < nacc) {
+    if (F.precision == RCHOL_PREC_FP32) P.acck32.alloc(nacc);
+    else P.acck64.alloc(nacc);
+  }
   P.kbuilt = true;
 }
 
