@@ -356,6 +356,17 @@ __global__ void __launch_bounds__(32) blk_invert_kernel(const BlkRec *recs, BlkI
 
 // ---- solving ----------------------------------------------------------------------------------
 
+// A solve is a chain of short kernels (two per tree depth and direction), so
+// each may start while the one before it still runs (programmatic dependent
+// launch): it sets up its barriers and loads what the plan holds, then waits
+// here until the kernels before it are complete and their writes visible.  It
+// must not touch vectors before that, and reads them with plain loads: the
+// compiler may move read-only ones above the wait.  The next kernel's start is
+// allowed as soon as all of this one's thread blocks run, so none of them ever
+// waits for room that a waiting kernel holds.
+__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // acc_i = in_i - (entries of row i in a CSR of external ones) out, LANES
 // lanes per row, four entries in flight per lane; in may be acc.  One
 // right-hand side (KC = 1), or columns (n apart) KC blockIdx.y and on of k, so
@@ -363,17 +374,22 @@ __global__ void __launch_bounds__(32) blk_invert_kernel(const BlkRec *recs, BlkI
 template <typename VT, typename InT, typename OutT, int LANES, int KC>
 __global__ void __launch_bounds__(256) blk_ext_kernel(const int32_t *__restrict__ rows, int64_t nrows,
                                                         const int64_t *__restrict__ rp, const int32_t *__restrict__ ci,
-                                                        const VT *__restrict__ v, const InT *in,
-                                                        const OutT *__restrict__ out, VT *acc, int k, int64_t n) {
+                                                        const VT *__restrict__ v, const InT *in, const OutT *out,
+                                                        VT *acc, int k, int64_t n) {
+  allow_next();
   const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LANES;
   const int sub = threadIdx.x % LANES, col0 = KC == 1 ? 0 : blockIdx.y * KC;
-  if (t >= nrows) return;  // whole groups leave together
-  const int64_t i = rows[t], q1 = rp[i + 1];
+  if (t >= nrows) {  // whole groups leave together
+    wait_previous();
+    return;
+  }
+  const int64_t i = rows[t], q0 = rp[i], q1 = rp[i + 1];
+  wait_previous();
   const OutT *oc[KC];
 #pragma unroll
   for (int j = 0; j < KC; ++j) oc[j] = KC == 1 ? out : out + min(col0 + j, k - 1) * n;
   VT s[KC][4] = {};
-  for (int64_t q = rp[i] + sub; q < q1; q += 4 * LANES) {
+  for (int64_t q = q0 + sub; q < q1; q += 4 * LANES) {
     int32_t c[4];
     VT w[4];
 #pragma unroll
@@ -565,7 +581,8 @@ __device__ __forceinline__ VT ext_sum(uint32_t cols, uint32_t vals, uint32_t q, 
 // for in step s.  One block-wide barrier per step, which also carries a
 // failed wait.
 template <typename VT, typename InT, typename OutT, bool UPPER, int NV, bool CLUSTER>
-__global__ void __launch_bounds__(512) blk_solve_kernel(BlkArgs<VT> a, const InT *__restrict__ in, OutT *out) {
+__global__ void __launch_bounds__(512) blk_solve_kernel(BlkArgs<VT> a, const InT *in, OutT *out) {
+  allow_next();
   extern __shared__ __align__(16) unsigned char smem[];
   const int C = CLUSTER ? a.C : 1;
   const int rank = CLUSTER ? (int)(blockIdx.x % (unsigned)C) : 0;
@@ -745,6 +762,7 @@ __global__ void __launch_bounds__(512) blk_solve_kernel(BlkArgs<VT> a, const InT
       }
     };
     OutT *op = out + at;
+    wait_previous();
     if (!CLUSTER) {
       fetch();
       rhs = next_rhs();
@@ -820,6 +838,7 @@ __global__ void __launch_bounds__(512) blk_solve_kernel(BlkArgs<VT> a, const InT
       for (int o = L >> 1; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
       if (l == 0) ps[(s & 1) * nown + j] = r - sum;
     };
+    wait_previous();
     if (CLUSTER) {
       fetch();
       prepare(0);
@@ -1083,6 +1102,27 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
 
 constexpr int kMaxDevices = 128;
 
+// Launch of a kernel that calls wait_previous, in clusters of C thread blocks;
+// early: it may start before the kernel ahead of it has ended.
+template <typename... Params, typename... Args>
+void chain_launch(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, int C, bool early,
+                  cudaStream_t s, const Args &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = early;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)C;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = C > 1 ? 2 : 1;
+  RCHOL_CUDA(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
+}
+
 template <typename VT, typename InT, typename OutT, bool UPPER, int NV>
 void launch_stage(const BlkStage &S, const BlkArgs<VT> &a, const InT *in, OutT *out, cudaStream_t s) {
   auto *single = blk_solve_kernel<VT, InT, OutT, UPPER, NV, false>;
@@ -1097,22 +1137,25 @@ void launch_stage(const BlkStage &S, const BlkArgs<VT> &a, const InT *in, OutT *
     RCHOL_CUDA(cudaFuncSetAttribute(multi, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   });
   const unsigned threads = (unsigned)(S.B / S.C / 4 * S.gl + S.helpers);
-  if (S.C == 1) {
-    single<<<(unsigned)S.npieces * (unsigned)a.k, threads, S.smem, s>>>(a, in, out);
-  } else {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)S.npieces * (unsigned)a.k * (unsigned)S.C);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = S.smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)S.C;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    RCHOL_CUDA(cudaLaunchKernelEx(&cfg, multi, a, in, out));
-  }
+  const unsigned blocks = (unsigned)S.npieces * (unsigned)a.k * (unsigned)S.C;
+  // A stage that starts early finds SMs busy with the one before, and its
+  // thread blocks would share the free ones while others stay empty later (in
+  // FP64, where an SM's arithmetic is what a step waits for, 700^2 took 1007 us
+  // instead of 728).  So a stage that fits the GPU in `waves` thread blocks per
+  // SM asks for the shared memory that admits no more.  Preconditioner, one
+  // right-hand side, starting in turn -> early -> early with this rule, us:
+  // FP32 80^3 547, 479, 444; 700^2 343, 273, 257; FP64 80^3 1283, 1354, 1199;
+  // 700^2 728, 1007, 644; 12^3 72, 47, 48.  FP64 stages of more than one wave
+  // start in turn: they run long, and early ones were up to 4% slower (700^2
+  // with 5 columns 1534 -> 1594 us).
+  const int side[] = {152, 76, 36, 15, 7};  // clusters of 1, 2, 4, 8, 16 that fit, one thread block per SM
+  const int fit = side[S.C == 1 ? 0 : S.C == 2 ? 1 : S.C == 4 ? 2 : S.C == 8 ? 3 : 4];
+  const int64_t waves = ((int64_t)S.npieces * a.k + fit - 1) / fit;
+  const bool early = sizeof(VT) == 4 || waves == 1;
+  size_t smem = S.smem;
+  if (early && waves <= 4) smem = std::max(smem, kBlkSmem / 16 / (size_t)(waves + 1) * 16 + 2048);
+  if (S.C == 1) chain_launch(single, blocks, threads, smem, 1, early, s, a, in, out);
+  else chain_launch(multi, blocks, threads, smem, S.C, early, s, a, in, out);
   note_launch();
   RCHOL_CUDA(cudaGetLastError());
 }
@@ -1140,9 +1183,9 @@ void launch_ext_kc(const BlkExt &E, int lanes, const int32_t *rows, int64_t nrow
                    VT *acc, int k, int64_t n, cudaStream_t s) {
   const dim3 grid((unsigned)((nrows * lanes + 255) / 256), (unsigned)((k + KC - 1) / KC));
   const VT *v = ext_values<VT>(E);
-  if (lanes == 2) blk_ext_kernel<VT, InT, OutT, 2, KC><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
-  else if (lanes == 8) blk_ext_kernel<VT, InT, OutT, 8, KC><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
-  else blk_ext_kernel<VT, InT, OutT, 32, KC><<<grid, 256, 0, s>>>(rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
+  if (lanes == 2) chain_launch(blk_ext_kernel<VT, InT, OutT, 2, KC>, grid, 256, 0, 1, true, s, rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
+  else if (lanes == 8) chain_launch(blk_ext_kernel<VT, InT, OutT, 8, KC>, grid, 256, 0, 1, true, s, rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
+  else chain_launch(blk_ext_kernel<VT, InT, OutT, 32, KC>, grid, 256, 0, 1, true, s, rows, nrows, E.rp.p, E.ci.p, v, in, out, acc, k, n);
   note_launch();
   RCHOL_CUDA(cudaGetLastError());
 }
