@@ -564,7 +564,7 @@ __device__ __forceinline__ VT ext_sum(uint32_t cols, uint32_t vals, uint32_t q, 
 // (product) and the shuffles of two sums.  Measured at 128^3 (FP32 forward,
 // the root's 16,384 rows, 32 steps of 512 by 16 thread blocks): 48 us, against
 // 293 us for 512 steps of 32 rows by one thread block (pipe_kernel); all
-// stages 507 us against 1122 us.  The subdomains (512 pieces, 92% of the
+// stages 507 us in turn, 455 us with early starts, against 1122 us.  The subdomains (512 pieces, 92% of the
 // rows) take 132 us of it for 490 MB, 3.7 TB/s (w2_kernel: 200 us).
 //   row threads: gl lanes per group of four own rows, a quarter of them per
 //     row for the sparse sums.  Step s adds the row's entries in block s-1 to
@@ -876,8 +876,8 @@ namespace {
 // costs about 1.3 us in a cluster (two exchanges, two barriers) whatever B
 // is, against about 1 us in a single thread block.  Short pieces take smaller
 // clusters: below maxrows the steps saved do not pay for the exchanges.
-// 128^3 log-normal, 512 subdomains, FP32 forward solve: 507 us with these
-// lines; 528 with clusters of 8 only up to 9 pieces, 527 with single thread
+// 128^3 log-normal, 512 subdomains, FP32 forward solve, kernels in turn: 507 us
+// with these lines; 528 with clusters of 8 only up to 9 pieces, 527 with single thread
 // blocks from 40 pieces on, 1122 with the record streams of trsv.cu.
 // In FP64 (2 FMA per clock and SM) the inverse's B / 2 products per row are
 // what a step costs, so B is smaller: 417 us for 64^3 with 64 subdomains
@@ -1033,13 +1033,20 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
       D.steps += (S.maxrows + S.B - 1) / S.B;
     }
     if (refit) continue;
+    int64_t slack = 0;  // the kernel loads one block past a piece's last
+    for (const BlkStage &S : D.stages) slack = std::max(slack, S.C * S.stride);
+    // Where the record streams solve too (FP32) or there is another plan
+    // already (several columns), memory that is short is left to what has no
+    // substitute.
+    size_t room = 0, total = 0;
+    RCHOL_CUDA(cudaMemGetInfo(&room, &total));
+    const size_t need = (size_t)off[nrec] + (size_t)(ninv + slack) * sizeof(VT) + (size_t)v.n * (sizeof(VT) + 4);
+    if (need > room / (sizeof(VT) == 4 || cols > 1 ? 8 : 2)) return false;
     D.rec_off.upload(off.data(), nrec + 1, s);
     D.recs.alloc(off[nrec]);
     blk_fill_kernel<VT><<<(unsigned)nrec, 128, 0, s>>>(d_recs.p, D.rec_off.p, d_cnt.p, rp.p, ci.p, v.p, bnd.p, upper,
                                                       early.p, nearly.p, D.recs.p);
     RCHOL_CUDA(cudaGetLastError());
-    int64_t slack = 0;  // the kernel loads one block past a piece's last
-    for (const BlkStage &S : D.stages) slack = std::max(slack, S.C * S.stride);
     inv.alloc(ninv + slack);
     RCHOL_CUDA(cudaMemsetAsync(inv.p, 0, inv.bytes(), s));
     RCHOL_CUDA(cudaFuncSetAttribute(blk_invert_kernel<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 256));
@@ -1229,11 +1236,15 @@ void launch_dir(const BlkDir &D, const VT *inv, const InT *in, OutT *out, VT *ac
 }
 
 bool build_block_dirs(const rchol_factor_s &F, int cols, BlkDir &fwd, BlkDir &bwd, cudaStream_t s) {
+  bool ok;
   if (F.precision == RCHOL_PREC_FP32)
-    return build_dir<float>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv32, s) &&
-           build_dir<float>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv32, s);
-  return build_dir<double>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv64, s) &&
+    ok = build_dir<float>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv32, s) &&
+         build_dir<float>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv32, s);
+  else
+    ok = build_dir<double>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv64, s) &&
          build_dir<double>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv64, s);
+  if (!ok) fwd = BlkDir(), bwd = BlkDir();  // no memory for half a plan
+  return ok;
 }
 
 }  // namespace
