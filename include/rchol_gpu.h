@@ -136,9 +136,8 @@ int rchol_gpu_factor_pivots(rchol_factor_t G, double *d);
  * block steps on the critical path (32 to 512 rows each).  No counterpart in
  * the reference. */
 int rchol_gpu_factor_plan_info(rchol_factor_t G, int transpose, int64_t *stages, int64_t *pieces, int64_t *steps);
-/* Autotuning of the preconditioner that PCG applies with this factor (with G
- * in FP64 there are no launch choices: it is timed and nothing changes):
- * times the preconditioner with alternative launch choices (L2 prefetch distance and ring depth of the
+/* Autotuning of the preconditioner that PCG applies with this factor: times it
+ * with alternative launch choices (L2 prefetch distance and ring depth of the
  * pipeline format, warps per thread block and prefetch of the warp format)
  * and keeps the fastest for all later solves with G.  ms_before / ms_after:
  * preconditioner time with the choices on entry / chosen; knobs (4 ints, may

@@ -43,7 +43,6 @@ void check_solve_status(cudaStream_t s);
 void wait_selftest(uint32_t polls, cudaStream_t s);
 void edge_grad(int64_t m, const int64_t *ei, const int64_t *ej, const double *lam, const double *x, double *g,
                cudaStream_t s);
-std::pair<double, double> tune_plan(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
 void precond_noalloc(const rchol_factor_s &F, const double *r, double *z, cudaStream_t s);
 
 }  // namespace rchol
@@ -283,7 +282,7 @@ int rchol_gpu_factor_tune(rchol_factor_t G, double *ms_before, double *ms_after,
   API_BEGIN
   RCHOL_CHECK_ARG(G && G->plan, "null factor");
   std::lock_guard<std::mutex> guard(G->plan->lock);
-  const std::pair<double, double> t = tune_plan(*G, *G->plan, 0);
+  const std::pair<double, double> t = tune_solves(*G, *G->plan, 0);
   if (ms_before) *ms_before = t.first;
   if (ms_after) *ms_after = t.second;
   if (knobs) {

@@ -196,7 +196,7 @@ struct SolvePlan {
   std::vector<std::unique_ptr<PcgWork>> pcg;
   std::vector<std::unique_ptr<SegWork>> seg;
   unsigned int *status = nullptr;  // status word of the solve kernels
-  bool blocked = false;    // the solves run on bfwd / bbwd (else, and in an FP32 PCG, on the record streams)
+  bool blocked = false;    // trsv and precond run on bfwd / bbwd (else, and in PCG, on the record streams)
   BlkDir bfwd, bbwd;
   BlkDir bkfwd, bkbwd;     // shapes for several right-hand sides (built on first use)
   bool kblocks = false, kwide = false;  // that was tried; it is there

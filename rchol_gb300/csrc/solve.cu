@@ -451,26 +451,25 @@ void build_plan(rchol_factor_s &F, cudaStream_t s) {
   auto P = new SolvePlan();
   try {
     P->status = solve_status_word();
-    // The solves run in large blocks (blocks.cu) where G allows it and
-    // RCHOL_TRSV_FORMAT does not ask for one of trsv.cu's record formats.  A
-    // PCG with G in FP32 stays with the record streams: its iterates follow
-    // the FP32 rounding of the preconditioner (of 40 systems solved to 1e-8
-    // five took an iteration more or less with another order of the sums), so
-    // a solve gives the same iterates as ever.  Both plans are then built at
-    // once, the records by the host's threads and the blocks by the GPU.
-    const bool blocks = !getenv("RCHOL_TRSV_FORMAT"), fp32 = F.precision == RCHOL_PREC_FP32;
+    // rchol_gpu_trsv_d and rchol_gpu_precond_d run in large blocks (blocks.cu)
+    // where G allows it and RCHOL_TRSV_FORMAT does not ask for one of trsv.cu's
+    // record formats.  The PCG loops always apply the record streams: CG
+    // amplifies the rounding of the preconditioner, so another order of its
+    // sums changes iteration counts (of 40 FP32 systems solved to 1e-8 five
+    // took an iteration more or less, of 15 FP64 ones two, with x off by
+    // 2e-9), and the same program has to give the same iterates as ever.  Both
+    // plans are built at once, the records by the host's threads and the
+    // blocks by the GPU.
     std::future<bool> other;
-    if (blocks && fp32) {
+    if (!getenv("RCHOL_TRSV_FORMAT")) {
       int dev = 0;
       RCHOL_CUDA(cudaGetDevice(&dev));
       other = std::async(std::launch::async, [&F, P, s, dev] {
         RCHOL_CUDA(cudaSetDevice(dev));
         return build_blocks(F, *P, s);
       });
-    } else {
-      P->blocked = blocks && build_blocks(F, *P, s);
     }
-    if (fp32 || !P->blocked) build_streams(F, *P, s);
+    build_streams(F, *P, s);
     if (other.valid()) P->blocked = other.get();
   } catch (...) {
     delete P;
@@ -599,7 +598,8 @@ static void blocks_k(const rchol_factor_s &F, const SolvePlan &P, int dir, const
   }
 }
 
-// The preconditioner with the plan's buffers already sized (inside PCG).
+// The preconditioner with the plan's buffers already sized: on the block plan
+// or the record streams (PCG: always these, see build_plan).
 static void precond_ready(const rchol_factor_s &F, bool blocks, const double *r, double *z, int k, cudaStream_t s);
 
 void trsv(const rchol_factor_s &F, bool upper, const double *in, double *out, int k, cudaStream_t s) {
@@ -620,9 +620,6 @@ void precond(const rchol_factor_s &F, const double *r, double *z, int k, cudaStr
   ensure_k(F, P.blocked, k, s);
   precond_ready(F, P.blocked, r, z, k, s);
 }
-
-// The preconditioner of the PCG loops (see build_plan).
-static bool pcg_blocks(const rchol_factor_s &F) { return F.plan->blocked && F.precision != RCHOL_PREC_FP32; }
 
 static void precond_ready(const rchol_factor_s &F, bool blocks, const double *r, double *z, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
@@ -701,35 +698,6 @@ void precond_noalloc(const rchol_factor_s &F, const double *r, double *z, cudaSt
   void *y = base + acc_bytes;
   precond_one(F, *F.plan, F.plan->blocked, r, z, fp32 ? nullptr : static_cast<double *>(y), fp32 ? static_cast<float *>(y) : nullptr,
               base, s);
-}
-
-// rchol_gpu_factor_tune: the launch choices of the preconditioner that PCG
-// applies.  The block plan has none: it is timed and left as it is.
-std::pair<double, double> tune_plan(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
-  if (!pcg_blocks(F)) return tune_solves(F, P, s);
-  const int64_t n = F.n;
-  const bool fp32 = F.precision == RCHOL_PREC_FP32;
-  DevBuf<double> r(n), z(n), y64(fp32 ? 0 : n);
-  DevBuf<float> y32(fp32 ? n : 0);
-  void *acc = ensure_acc(P, fp32, n);
-  RCHOL_CUDA(cudaMemsetAsync(r.p, 0, r.bytes(), s));
-  cudaEvent_t e0, e1;
-  RCHOL_CUDA(cudaEventCreate(&e0));
-  RCHOL_CUDA(cudaEventCreate(&e1));
-  float best = 1e30f;
-  for (int rep = 0; rep < 4; ++rep) {
-    RCHOL_CUDA(cudaEventRecord(e0, s));
-    precond_one(F, P, true, r.p, z.p, y64.p, y32.p, acc, s);
-    RCHOL_CUDA(cudaEventRecord(e1, s));
-    RCHOL_CUDA(cudaEventSynchronize(e1));
-    float ms = 0.f;
-    RCHOL_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    if (rep) best = std::min(best, ms);
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  P.tuned_ms = best;
-  return {best, best};
 }
 
 void spmv_public(const rchol_matrix_s &A, const double *x, double *y, int k, cudaStream_t s) {
@@ -853,7 +821,7 @@ static void pcg_iteration(const rchol_matrix_s &A, const rchol_factor_s &F, PcgW
   const int k = w.k;
   const int64_t n = A.n, nk = n * k;
   const unsigned eb = (unsigned)((nk + 255) / 256);
-  precond_ready(F, pcg_blocks(F), w.r.p, w.z.p, k, s);
+  precond_ready(F, false, w.r.p, w.z.p, k, s);
   reduce_kernel<RED_DOT><<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, st, w.r.p, w.z.p, nullptr, nullptr, nullptr);
   finalize_kernel<<<k, RED_THREADS, 0, s>>>(st, FIN_BETA, 0, nullptr);
   pupdate_kernel<<<eb, 256, 0, s>>>(nk, st, w.p.p, w.z.p);
@@ -876,7 +844,7 @@ static void pcg_impl(const rchol_matrix_s &A, const rchol_factor_s &F, const dou
   const int64_t n = A.n, nk = n * k;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   ensure_scratch(P, fp32, nk);
-  ensure_k(F, pcg_blocks(F), k, s);
+  ensure_k(F, false, k, s);
   PcgWork &w = pcg_workspace(A, F, k);
   PcgState st = pcg_state(w);
   cudaStream_t ws = w.stream;
@@ -1249,7 +1217,7 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
     cudaGraph_t g = nullptr;
     RCHOL_CUDA(cudaStreamBeginCapture(ws, cudaStreamCaptureModeThreadLocal));
     try {
-      precond_ready(F, pcg_blocks(F), w.r.p, w.z.p, 1, ws);
+      precond_ready(F, false, w.r.p, w.z.p, 1, ws);
       const unsigned C = S * SEG_GROUPS;
       // element updates: enough parts of a system for four thread blocks an SM
       const dim3 E(S, std::min(64u, (4 * seg_sms() + S - 1) / S));

@@ -1,5 +1,5 @@
 // Block triangular solves with G (forward) and G^T (backward) from streams of
-// 32-row records: PCG with G in FP32, factors whose rows are too dense for the
+// 32-row records: PCG, factors whose rows are too dense for the
 // large blocks of blocks.cu or whose entries have mixed signs, and the formats
 // that RCHOL_TRSV_FORMAT names.
 //
