@@ -131,10 +131,10 @@ int rchol_gpu_factor_precision(rchol_factor_t G);
 int rchol_gpu_factor_export(rchol_factor_t G, int64_t *row_ptr, int64_t *col_idx, double *val);
 /* Pivots d of the factorization (length n), G = L sqrt(D). */
 int rchol_gpu_factor_pivots(rchol_factor_t G, double *d);
-/* Shape of the triangular-solve plan of the forward (transpose = 0) or
- * backward solve: stages (kernels in sequence), pieces, and the sequential
- * block steps on the critical path (32 to 512 rows each).  No counterpart in
- * the reference. */
+/* Shape of the triangular-solve plan that PCG applies, of the forward
+ * (transpose = 0) or backward solve: stages (kernel pairs in sequence),
+ * pieces, and the sequential 32-row block steps on the critical path.  No
+ * counterpart in the reference. */
 int rchol_gpu_factor_plan_info(rchol_factor_t G, int transpose, int64_t *stages, int64_t *pieces, int64_t *steps);
 /* Autotuning of the preconditioner that PCG applies with this factor: times it
  * with alternative launch choices (L2 prefetch distance and ring depth of the

@@ -1003,7 +1003,6 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
     RCHOL_CUDA(cudaStreamSynchronize(s));
     std::vector<int64_t> off(nrec + 1, 0);
     bool refit = false;
-    D.steps = 0;
     for (size_t st = 0; st < D.stages.size(); ++st) {
       BlkStage &S = D.stages[st];
       int64_t maxrec = 0, late = 0;
@@ -1030,7 +1029,6 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
       const int most = 6;
       while (S.ring < most && stage_smem(S, sizeof(VT), S.ring + 1) <= (S.C > 1 ? kBlkSmem / 2 : kBlkSmem / 4)) ++S.ring;
       S.smem = stage_smem(S, sizeof(VT), S.ring);
-      D.steps += (S.maxrows + S.B - 1) / S.B;
     }
     if (refit) continue;
     int64_t slack = 0;  // the kernel loads one block past a piece's last
@@ -1064,7 +1062,6 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
       RCHOL_CUDA(cudaGetLastError());
     }
     D.pieces.upload(pieces.data(), pieces.size(), s);
-    D.npieces = (int64_t)pieces.size();
     D.early_rows = 0;
     if (early.p) {
       std::vector<int32_t> rows;

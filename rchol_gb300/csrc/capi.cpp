@@ -264,13 +264,6 @@ int64_t rchol_gpu_factor_nnz(rchol_factor_t G) { return G ? G->nnz : -1; }
 int rchol_gpu_factor_plan_info(rchol_factor_t G, int transpose, int64_t *stages, int64_t *pieces, int64_t *steps) {
   API_BEGIN
   RCHOL_CHECK_ARG(G && G->plan, "null factor");
-  if (G->plan->blocked) {
-    const BlkDir &B = transpose ? G->plan->bbwd : G->plan->bfwd;
-    if (stages) *stages = (int64_t)B.stages.size();
-    if (pieces) *pieces = B.npieces;
-    if (steps) *steps = B.steps;
-    return RCHOL_OK;
-  }
   const StreamDir &D = transpose ? G->plan->sbwd : G->plan->sfwd;
   if (stages) *stages = (int64_t)D.stage_ptr.size() - 1;
   if (pieces) *pieces = D.stage_ptr.empty() ? 0 : D.stage_ptr.back();

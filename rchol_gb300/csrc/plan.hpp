@@ -133,7 +133,6 @@ struct BlkDir {
   BlkExt early, late;
   DevBuf<int32_t> erow;  // the later stages' rows
   int64_t early_rows = 0;
-  int64_t steps = 0, npieces = 0;
 };
 
 // Workspace and captured CUDA graph of one PCG iteration for a given matrix

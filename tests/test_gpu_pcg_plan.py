@@ -73,3 +73,14 @@ def test_gradient(cuda, R, monkeypatch):
         return x.detach(), w.grad, b.grad
 
     assert all(torch.equal(p, q) for p, q in zip(*_both(monkeypatch, solve)))
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
+def test_plan_info(cuda, R, monkeypatch, precision):
+    """The reported plan is the one PCG applies."""
+    A = generators.laplace_3d(24)
+    tree = R.Tree.build(A.indptr, A.indices, 16)
+    Ad = R.Matrix.create(A.indptr, A.indices, A.data, tree)
+    own, streams = _both(monkeypatch, lambda: R.Factor.compute(Ad, tree, seed=5, precision=precision))
+    for transpose in (False, True):
+        assert own.plan_info(transpose) == streams.plan_info(transpose)
