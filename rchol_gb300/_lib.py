@@ -51,6 +51,7 @@ SIGNATURES = [
     ("rchol_gpu_factor_levels", C.c_int, [_vp, _i64p, _i64p]),
     ("rchol_gpu_factor_setup_times", C.c_int, [_vp, _dp, _dp, _dp]),
     ("rchol_gpu_factor_plan_info", C.c_int, [_vp, C.c_int, _i64p, _i64p, _i64p]),
+    ("rchol_gpu_factor_blocked", C.c_int, [_vp]),
     ("rchol_gpu_factor_tune", C.c_int, [_vp, _dp, _dp, C.POINTER(C.c_int)]),
     ("rchol_gpu_factor_destroy", None, [_vp]),
     ("rchol_gpu_pcg", C.c_int, [_vp, _vp, _dp, _dp, _i64, C.c_double, C.c_int, _dp, _ip]),
@@ -260,6 +261,10 @@ class Factor(Handle):
         a, b, c = _i64(), _i64(), _i64()
         check(lib().rchol_gpu_factor_plan_info(self.ptr, int(transpose), C.byref(a), C.byref(b), C.byref(c)))
         return a.value, b.value, c.value
+
+    def blocked(self):
+        """Whether trsv and precond solve in large blocks."""
+        return bool(lib().rchol_gpu_factor_blocked(self.ptr))
 
     def tune(self):
         """Times the solves with alternative launch choices on this factor and

@@ -1033,13 +1033,15 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
     if (refit) continue;
     int64_t slack = 0;  // the kernel loads one block past a piece's last
     for (const BlkStage &S : D.stages) slack = std::max(slack, S.C * S.stride);
-    // Where the record streams solve too (FP32) or there is another plan
-    // already (several columns), memory that is short is left to what has no
-    // substitute.
+    // A plan of over an eighth of the device's memory per direction is left
+    // out: the record streams (for several columns, the first plan) solve too.
+    // The line is drawn by the problem alone, not by what is free just now:
+    // the two plans round differently, and a program's results must not
+    // depend on what else is resident.
     size_t room = 0, total = 0;
     RCHOL_CUDA(cudaMemGetInfo(&room, &total));
     const size_t need = (size_t)off[nrec] + (size_t)(ninv + slack) * sizeof(VT) + (size_t)v.n * (sizeof(VT) + 4);
-    if (need > room / (sizeof(VT) == 4 || cols > 1 ? 8 : 2)) return false;
+    if (need > total / 8) return false;
     D.rec_off.upload(off.data(), nrec + 1, s);
     D.recs.alloc(off[nrec]);
     blk_fill_kernel<VT><<<(unsigned)nrec, 128, 0, s>>>(d_recs.p, D.rec_off.p, d_cnt.p, rp.p, ci.p, v.p, bnd.p, upper,
@@ -1232,24 +1234,36 @@ void launch_dir(const BlkDir &D, const VT *inv, const InT *in, OutT *out, VT *ac
   }
 }
 
-bool build_block_dirs(const rchol_factor_s &F, int cols, BlkDir &fwd, BlkDir &bwd, cudaStream_t s) {
-  bool ok;
-  if (F.precision == RCHOL_PREC_FP32)
-    ok = build_dir<float>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv32, s) &&
-         build_dir<float>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv32, s);
-  else
-    ok = build_dir<double>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv64, s) &&
-         build_dir<double>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv64, s);
-  if (!ok) fwd = BlkDir(), bwd = BlkDir();  // no memory for half a plan
-  return ok;
+// make() builds into fwd and bwd; kNoMemory where an allocation failed (the
+// record streams or the first plan solve without this one).  Half a plan is
+// given back.
+template <typename Make>
+BlkBuilt try_build(BlkDir &fwd, BlkDir &bwd, Make make) {
+  BlkBuilt built = BlkBuilt::kLeftOut;
+  try {
+    if (make()) return BlkBuilt::kReady;
+  } catch (const Error &e) {
+    if (e.status != RCHOL_ERR_NOMEM) throw;
+    (void)cudaGetLastError();  // the failed allocation's
+    built = BlkBuilt::kNoMemory;
+  }
+  fwd = BlkDir();
+  bwd = BlkDir();
+  return built;
 }
 
-}  // namespace
+bool build_block_dirs(const rchol_factor_s &F, int cols, BlkDir &fwd, BlkDir &bwd, cudaStream_t s) {
+  if (F.precision == RCHOL_PREC_FP32)
+    return build_dir<float>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv32, s) &&
+           build_dir<float>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv32, s);
+  return build_dir<double>(F.n, F.lrp, F.lci, F.lv, F.nodes, false, cols, fwd, fwd.inv64, s) &&
+         build_dir<double>(F.n, F.urp, F.uci, F.uv, F.nodes, true, cols, bwd, bwd.inv64, s);
+}
 
-bool build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
-  // Inverses of large triangles are as accurate as substitution because
-  // nothing cancels in them: the diagonal is positive and no other entry is
-  // (true of every sampled factor).  Any other G keeps the record streams.
+// Inverses of large triangles are as accurate as substitution because nothing
+// cancels in them: the diagonal is positive and no other entry is (true of
+// every sampled factor).  Any other G keeps the record streams.
+bool block_signs(const rchol_factor_s &F, cudaStream_t s) {
   DevBuf<unsigned long long> positive(2);
   RCHOL_CUDA(cudaMemsetAsync(positive.p, 0, positive.bytes(), s));
   blk_sign_kernel<<<1024, 256, 0, s>>>(F.n, F.nnz, F.urp.p, F.uv.p, positive.p);
@@ -1257,13 +1271,19 @@ bool build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
   unsigned long long count[2];
   positive.download(count, 2, s);
   RCHOL_CUDA(cudaStreamSynchronize(s));
-  if (count[0] != (unsigned long long)F.n || count[1] != (unsigned long long)F.n) return false;
-  return build_block_dirs(F, 1, P.bfwd, P.bbwd, s);
+  return count[0] == (unsigned long long)F.n && count[1] == (unsigned long long)F.n;
+}
+
+}  // namespace
+
+BlkBuilt build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
+  return try_build(P.bfwd, P.bbwd, [&] { return block_signs(F, s) && build_block_dirs(F, 1, P.bfwd, P.bbwd, s); });
 }
 
 void build_blocks_k(const rchol_factor_s &F, SolvePlan &P, int k, cudaStream_t s) {
   if (P.kblocks || k < kBlkWideFrom) return;
-  P.kwide = build_block_dirs(F, kBlkWideCols, P.bkfwd, P.bkbwd, s);
+  P.kwide = try_build(P.bkfwd, P.bkbwd, [&] { return build_block_dirs(F, kBlkWideCols, P.bkfwd, P.bkbwd, s); }) ==
+            BlkBuilt::kReady;
   P.kblocks = true;
 }
 

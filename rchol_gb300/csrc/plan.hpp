@@ -212,8 +212,10 @@ struct SolvePlan {
   DevBuf<double> colk;     // right-hand sides and solutions column after column
 };
 
-// Block plan of both directions; false if G's rows are too dense for it.
-bool build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
+// Block plan of both directions.  Left out: G's rows are too dense for it, its
+// entries have mixed signs, or it would be too large.
+enum class BlkBuilt { kReady, kLeftOut, kNoMemory };
+BlkBuilt build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
 // The plan that k right-hand sides take, where it is another one.
 void build_blocks_k(const rchol_factor_s &F, SolvePlan &P, int k, cudaStream_t s);
 // Solve with G (upper = false) or G^T for k <= kBlkCols right-hand sides, one

@@ -459,9 +459,12 @@ void build_plan(rchol_factor_s &F, cudaStream_t s) {
     // took an iteration more or less, of 15 FP64 ones two, with x off by
     // 2e-9), and the same program has to give the same iterates as ever.  Both
     // plans are built at once, the records by the host's threads and the
-    // blocks by the GPU.
-    std::future<bool> other;
-    if (!getenv("RCHOL_TRSV_FORMAT")) {
+    // blocks by the GPU.  Where memory is too short for that, the streams are
+    // built alone and the block plan after them if it still fits.
+    const bool wanted = !getenv("RCHOL_TRSV_FORMAT");
+    BlkBuilt built = BlkBuilt::kLeftOut;
+    std::future<BlkBuilt> other;
+    if (wanted) {
       int dev = 0;
       RCHOL_CUDA(cudaGetDevice(&dev));
       other = std::async(std::launch::async, [&F, P, s, dev] {
@@ -469,8 +472,22 @@ void build_plan(rchol_factor_s &F, cudaStream_t s) {
         return build_blocks(F, *P, s);
       });
     }
-    build_streams(F, *P, s);
-    if (other.valid()) P->blocked = other.get();
+    try {
+      build_streams(F, *P, s);
+      if (wanted) built = other.get();
+    } catch (const Error &e) {
+      if (!wanted || e.status != RCHOL_ERR_NOMEM) throw;
+      (void)cudaGetLastError();
+      if (other.valid()) other.wait();
+      P->bfwd = BlkDir();
+      P->bbwd = BlkDir();
+      P->sfwd = StreamDir();
+      P->sbwd = StreamDir();
+      build_streams(F, *P, s);
+      built = BlkBuilt::kNoMemory;
+    }
+    if (built == BlkBuilt::kNoMemory) built = build_blocks(F, *P, s);
+    P->blocked = built == BlkBuilt::kReady;
   } catch (...) {
     delete P;
     throw;
