@@ -135,6 +135,15 @@ struct BlkDir {
   int64_t early_rows = 0;
 };
 
+// Vectors of solves on the block plan with up to `cols` right-hand sides:
+// right-hand sides and solutions column after column (cols > 1), and what lies
+// between the two solves of the preconditioner.
+struct BlkWork {
+  int cols = 0;
+  DevBuf<double> a, b, y64;
+  DevBuf<float> y32;
+};
+
 // Workspace and captured CUDA graph of one PCG iteration for a given matrix
 // and number of right-hand sides (solve.cu).
 struct PcgWork {
@@ -209,7 +218,7 @@ struct SolvePlan {
   DevBuf<float> acc32;
   DevBuf<double> acck64;   // the same for up to 32 right-hand sides (n x 32)
   DevBuf<float> acck32;
-  DevBuf<double> colk;     // right-hand sides and solutions column after column
+  std::vector<BlkWork> work;  // of the block plan; the last is in use
 };
 
 // Block plan of both directions.  Left out: G's rows are too dense for it, its

@@ -537,28 +537,39 @@ static void *ensure_acc(SolvePlan &P, bool fp32, int64_t n) {
   return P.acc64.p;
 }
 
-// What k right-hand sides need beyond ensure_scratch, on the block plan or the
-// record streams.
-static void ensure_k(const rchol_factor_s &F, bool blocks, int k, cudaStream_t s) {
+// What k right-hand sides need on the record streams.
+static void ensure_streams(const rchol_factor_s &F, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  ensure_scratch(P, fp32, F.n * k);
+  if (k == 1) ensure_acc(P, fp32, F.n);
+  else build_streams_k(F, P, s);
+}
+
+// What k right-hand sides need on the block plan.  Columns come in a power of
+// two.  A workspace that is grown out of stays until the factor goes, because
+// a caller's graph of a solve with fewer columns holds its addresses (all of
+// them together are smaller than the last).
+static void ensure_blocks(const rchol_factor_s &F, int k, cudaStream_t s) {
+  SolvePlan &P = *F.plan;
+  const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  const size_t n = (size_t)F.n;
+  int cols = 1;
+  while (cols < std::min(k, kBlkCols)) cols *= 2;
   if (k == 1) {
     ensure_acc(P, fp32, F.n);
-    return;
+  } else {
+    build_blocks_k(F, P, std::min(k, kBlkCols), s);
+    if (fp32 && P.acck32.n < n * kBlkCols) P.acck32.alloc(n * kBlkCols);
+    if (!fp32 && P.acck64.n < n * kBlkCols) P.acck64.alloc(n * kBlkCols);
   }
-  if (!blocks) {
-    build_streams_k(F, P, s);
-    return;
-  }
-  build_blocks_k(F, P, std::min(k, kBlkCols), s);
-  const size_t all = (size_t)F.n * kBlkCols, cols = 2 * (size_t)F.n * std::min(k, kBlkCols);
-  if (fp32 && P.acck32.n < all) P.acck32.alloc(all);
-  if (!fp32 && P.acck64.n < all) P.acck64.alloc(all);
-  if (P.colk.n < cols) {
-    P.colk.alloc(cols);
-    P.pcg.clear();  // their graphs hold the old address
-    P.seg.clear();
-  }
+  if (!P.work.empty() && P.work.back().cols >= cols) return;
+  BlkWork w;
+  w.cols = cols;
+  if (fp32) w.y32.alloc(n * cols);
+  else w.y64.alloc(n * cols);
+  if (cols > 1) w.a.alloc(n * cols), w.b.alloc(n * cols);
+  P.work.push_back(std::move(w));
 }
 
 // Columns j0 .. j0 + g of an n x k row-major array, one after another
@@ -597,34 +608,46 @@ static void blocks_k(const rchol_factor_s &F, const SolvePlan &P, int dir, const
   const int64_t n = F.n;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   void *acc = fp32 ? (void *)P.acck32.p : (void *)P.acck64.p;
-  double *a = P.colk.p;
+  const BlkWork &w = P.work.back();
+  double *a = w.a.p, *b = w.b.p;
   for (int j0 = 0; j0 < k; j0 += kBlkCols) {
     const int g = std::min(kBlkCols, k - j0);
-    double *b = a + n * g;
     move_columns<true>(n, k, j0, g, in, a, s);
     if (dir < 2) {
       block_trsv(F, P, dir == 1, a, nullptr, b, nullptr, acc, g, s);
     } else if (fp32) {
-      block_trsv(F, P, false, a, nullptr, nullptr, P.ytmp32.p, acc, g, s);
-      block_trsv(F, P, true, nullptr, P.ytmp32.p, b, nullptr, acc, g, s);
+      block_trsv(F, P, false, a, nullptr, nullptr, w.y32.p, acc, g, s);
+      block_trsv(F, P, true, nullptr, w.y32.p, b, nullptr, acc, g, s);
     } else {
-      block_trsv(F, P, false, a, nullptr, P.ytmp.p, nullptr, acc, g, s);
-      block_trsv(F, P, true, P.ytmp.p, nullptr, b, nullptr, acc, g, s);
+      block_trsv(F, P, false, a, nullptr, w.y64.p, nullptr, acc, g, s);
+      block_trsv(F, P, true, w.y64.p, nullptr, b, nullptr, acc, g, s);
     }
     move_columns<false>(n, k, j0, g, b, out, s);
   }
 }
 
-// The preconditioner with the plan's buffers already sized: on the block plan
-// or the record streams (PCG: always these, see build_plan).
-static void precond_ready(const rchol_factor_s &F, bool blocks, const double *r, double *z, int k, cudaStream_t s);
+// The preconditioner by the record streams, with the plan's buffers already
+// sized (inside PCG).
+static void precond_streams(const rchol_factor_s &F, const double *r, double *z, int k, cudaStream_t s) {
+  SolvePlan &P = *F.plan;
+  const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  if (k == 1) {
+    precond_one(F, P, false, r, z, P.ytmp.p, P.ytmp32.p, ensure_acc(P, fp32, F.n), s);
+  } else if (fp32) {
+    stream_trsv_k(F, P, false, r, nullptr, nullptr, P.ytmp32.p, k, s);
+    stream_trsv_k(F, P, true, nullptr, P.ytmp32.p, z, nullptr, k, s);
+  } else {
+    stream_trsv_k(F, P, false, r, nullptr, P.ytmp.p, nullptr, k, s);
+    stream_trsv_k(F, P, true, P.ytmp.p, nullptr, z, nullptr, k, s);
+  }
+}
 
 void trsv(const rchol_factor_s &F, bool upper, const double *in, double *out, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
-  ensure_scratch(P, fp32, F.n * k);
-  ensure_k(F, P.blocked, k, s);
+  if (P.blocked) ensure_blocks(F, k, s);
+  else ensure_streams(F, k, s);
   if (k == 1) trsv_one(F, P, P.blocked, upper, in, nullptr, out, nullptr, ensure_acc(P, fp32, F.n), s);
   else if (P.blocked) blocks_k(F, P, upper, in, out, k, s);
   else stream_trsv_k(F, P, upper, in, nullptr, out, nullptr, k, s);
@@ -633,25 +656,15 @@ void trsv(const rchol_factor_s &F, bool upper, const double *in, double *out, in
 void precond(const rchol_factor_s &F, const double *r, double *z, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
-  ensure_scratch(P, F.precision == RCHOL_PREC_FP32, F.n * k);
-  ensure_k(F, P.blocked, k, s);
-  precond_ready(F, P.blocked, r, z, k, s);
-}
-
-static void precond_ready(const rchol_factor_s &F, bool blocks, const double *r, double *z, int k, cudaStream_t s) {
-  SolvePlan &P = *F.plan;
-  const bool fp32 = F.precision == RCHOL_PREC_FP32;
-  if (k == 1) {
-    precond_one(F, P, blocks, r, z, P.ytmp.p, P.ytmp32.p, ensure_acc(P, fp32, F.n), s);
-  } else if (blocks) {
-    blocks_k(F, P, 2, r, z, k, s);
-  } else if (fp32) {
-    stream_trsv_k(F, P, false, r, nullptr, nullptr, P.ytmp32.p, k, s);
-    stream_trsv_k(F, P, true, nullptr, P.ytmp32.p, z, nullptr, k, s);
-  } else {
-    stream_trsv_k(F, P, false, r, nullptr, P.ytmp.p, nullptr, k, s);
-    stream_trsv_k(F, P, true, P.ytmp.p, nullptr, z, nullptr, k, s);
+  if (!P.blocked) {
+    ensure_streams(F, k, s);
+    precond_streams(F, r, z, k, s);
+    return;
   }
+  ensure_blocks(F, k, s);
+  const BlkWork &w = P.work.back();
+  if (k == 1) precond_one(F, P, true, r, z, w.y64.p, w.y32.p, ensure_acc(P, F.precision == RCHOL_PREC_FP32, F.n), s);
+  else blocks_k(F, P, 2, r, z, k, s);
 }
 
 // ---- preconditioner apply without allocation --------------------------------------------
@@ -838,7 +851,7 @@ static void pcg_iteration(const rchol_matrix_s &A, const rchol_factor_s &F, PcgW
   const int k = w.k;
   const int64_t n = A.n, nk = n * k;
   const unsigned eb = (unsigned)((nk + 255) / 256);
-  precond_ready(F, false, w.r.p, w.z.p, k, s);
+  precond_streams(F, w.r.p, w.z.p, k, s);
   reduce_kernel<RED_DOT><<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, st, w.r.p, w.z.p, nullptr, nullptr, nullptr);
   finalize_kernel<<<k, RED_THREADS, 0, s>>>(st, FIN_BETA, 0, nullptr);
   pupdate_kernel<<<eb, 256, 0, s>>>(nk, st, w.p.p, w.z.p);
@@ -859,9 +872,7 @@ static void pcg_impl(const rchol_matrix_s &A, const rchol_factor_s &F, const dou
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
   const int64_t n = A.n, nk = n * k;
-  const bool fp32 = F.precision == RCHOL_PREC_FP32;
-  ensure_scratch(P, fp32, nk);
-  ensure_k(F, false, k, s);
+  ensure_streams(F, k, s);
   PcgWork &w = pcg_workspace(A, F, k);
   PcgState st = pcg_state(w);
   cudaStream_t ws = w.stream;
@@ -1214,9 +1225,7 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
   const int64_t n = A.n;
-  const bool fp32 = F.precision == RCHOL_PREC_FP32;
-  ensure_scratch(P, fp32, n);
-  ensure_acc(P, fp32, n);
+  ensure_streams(F, 1, s);
   SegWork &w = seg_workspace(A, F, nseg, seg);
   SegState st = seg_state(w);
   const unsigned S = (unsigned)nseg;
@@ -1234,7 +1243,7 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
     cudaGraph_t g = nullptr;
     RCHOL_CUDA(cudaStreamBeginCapture(ws, cudaStreamCaptureModeThreadLocal));
     try {
-      precond_ready(F, false, w.r.p, w.z.p, 1, ws);
+      precond_streams(F, w.r.p, w.z.p, 1, ws);
       const unsigned C = S * SEG_GROUPS;
       // element updates: enough parts of a system for four thread blocks an SM
       const dim3 E(S, std::min(64u, (4 * seg_sms() + S - 1) / S));
