@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "common.hpp"
+#include "elim_shape.hpp"
 #include "host.hpp"
 
 namespace rchol {
@@ -60,7 +61,7 @@ struct PoolRec {
 };
 static_assert(sizeof(PoolRec) == 24, "PoolRec layout");
 
-enum { FLAG_FILL = 0, FLAG_WIDTH = 1, FLAG_GCAP = 2, FLAG_SINGULAR = 3, NFLAGS = 4 };
+enum { FLAG_FILL = 0, FLAG_GCAP = 1, FLAG_SINGULAR = 2, NFLAGS = 3 };  // then the widest column per depth
 
 struct ElimArgs {
   const int64_t *lrp;  // extended Laplacian, upper CSR
@@ -87,6 +88,7 @@ struct ElimArgs {
   int64_t gcap;
   double *diag;
   int *flags;
+  int *widest;               // records of the widest column of this depth that did not fit
   uint64_t seed;
   int emax;                  // per-warp buffer capacity in entries
   unsigned char *gscratch;   // per-warp buffers in HBM when they exceed shared memory
@@ -367,7 +369,7 @@ __global__ void eliminate_kernel(ElimArgs a) {
     }
     int total = ninit + (int)nall;
     if (total > E) {
-      if (lane == 0) atomicMax(&a.flags[FLAG_WIDTH], total);
+      if (lane == 0) atomicMax(a.widest, total);
       total = 0;  // skip the column; the host retries with wider buffers
     }
     // fill records: one 16-byte load each, two per lane in flight
@@ -693,7 +695,7 @@ __global__ void __launch_bounds__(EB) eliminate_block_kernel(ElimArgs a) {
     double *cval = ival + cur * E, *nval = ival + (cur ^ 1) * E;
     int n = s_n[cur];
     if (n > E) {
-      if (tid == 0) atomicMax(&a.flags[FLAG_WIDTH], n);
+      if (tid == 0) atomicMax(a.widest, n);
       n = 0;  // skip the column; the host retries with wider buffers
     }
     // ---- sort by (row, source); the last column's records are written -------
@@ -933,16 +935,6 @@ __global__ void u32_to_i64_kernel(int64_t n, const uint32_t *a, int64_t *b) {
 // Exclusive scan of int64 counts in place: out[0..n] with out[n] = total.
 void exclusive_scan_i64(int64_t *d_data, int64_t n, cudaStream_t s);
 
-namespace {
-
-int pow2_at_least(int x) {
-  int p = 32;
-  while (p < x) p <<= 1;
-  return p;
-}
-
-}  // namespace
-
 void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t seed,
                 rchol_factor_s &F, cudaStream_t s) {
   const int64_t next = ext.n, n = next - 1;
@@ -996,14 +988,15 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
   const size_t smem_limit = prop.sharedMemPerBlockOptin;
   RCHOL_CUDA(cudaFuncSetAttribute(eliminate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_limit));
-  const size_t block_limit = smem_limit - 2048;  // beside the static arrays
+  const size_t block_limit = smem_limit - 2048;  // beside the static arrays (see elim_shape)
   RCHOL_CUDA(cudaFuncSetAttribute(eliminate_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)block_limit));
   const int64_t pool_cap = std::max<int64_t>(1 << 16, next / 4);
 
   DevBuf<double> diag(next);
-  DevBuf<int> flags(NFLAGS);
-  int widest = 0;  // the widest column that did not fit a buffer so far
+  const int nflags = NFLAGS + maxdepth + 1;
+  DevBuf<int> flags(nflags);
+  std::vector<int> widest(maxdepth + 1, 0);  // per depth: the widest column that did not fit a buffer so far
   for (int attempt = 0; attempt < 12; ++attempt) {
     std::vector<int64_t> base(next + 1, 0);
     for (int64_t c = 0; c < next; ++c) base[c + 1] = base[c] + cap[c];
@@ -1051,37 +1044,16 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
     args.flags = flags.p;
     args.seed = seed;
     std::vector<DevBuf<int64_t>> keep;
+    const std::vector<int> width = depth_widths(coldepth, initdeg, cap, widest);
     for (int depth = maxdepth; depth >= 1; --depth) {
       std::vector<int64_t> nb, ne;
-      int width = std::max(32, widest);
       for (auto &nd : nodes) {
         if (nd.depth != depth || nd.end <= nd.begin) continue;
         nb.push_back(nd.begin);
         ne.push_back(nd.end);
-        for (int64_t c = nd.begin; c < nd.end; ++c)
-          width = std::max(width, initdeg[c] + (int)cap[c]);
       }
       if (nb.empty()) continue;
-      // four warps per node unless the nodes alone fill the GPU several times
-      const size_t block_bytes = (size_t)std::max(256, pow2_at_least(width)) * 96;
-      if ((int64_t)nb.size() <= 8 * (int64_t)prop.multiProcessorCount && block_bytes <= block_limit) {
-        keep.emplace_back(nb.size());
-        keep.back().upload(nb.data(), nb.size(), s);
-        keep.emplace_back(ne.size());
-        keep.back().upload(ne.data(), ne.size(), s);
-        args.node_begin = keep[keep.size() - 2].p;
-        args.node_end = keep.back().p;
-        args.num_nodes = (int)nb.size();
-        args.emax = std::max(256, pow2_at_least(width));
-        args.gscratch = nullptr;
-        eliminate_block_kernel<<<(unsigned)nb.size(), EB, block_bytes, s>>>(args);
-        RCHOL_CUDA(cudaGetLastError());
-        continue;
-      }
-      int emax = pow2_at_least(std::max(width, 128));
-      size_t per_warp = (size_t)emax * 40;
-      const bool in_smem = per_warp <= smem_limit;
-      int wpb = in_smem ? (int)std::min<size_t>(4, smem_limit / per_warp) : 1;
+      const ElimShape S = elim_shape(width[depth], (int64_t)nb.size(), prop.multiProcessorCount, smem_limit);
       keep.emplace_back(nb.size());
       keep.back().upload(nb.data(), nb.size(), s);
       keep.emplace_back(ne.size());
@@ -1089,20 +1061,28 @@ void gpu_factor(const HostCsr &ext, const std::vector<TreeNode> &nodes, uint64_t
       args.node_begin = keep[keep.size() - 2].p;
       args.node_end = keep.back().p;
       args.num_nodes = (int)nb.size();
-      args.emax = emax;
+      args.emax = S.emax;
+      args.widest = flags.p + NFLAGS + depth;
+      args.gscratch = nullptr;
+      if (S.four_warps) {
+        eliminate_block_kernel<<<(unsigned)nb.size(), EB, S.node_smem, s>>>(args);
+        RCHOL_CUDA(cudaGetLastError());
+        continue;
+      }
       DevBuf<unsigned char> wide;
-      if (!in_smem) wide.alloc(per_warp * nb.size());
+      if (!S.node_smem) wide.alloc((size_t)S.emax * 40 * nb.size());
       args.gscratch = wide.p;
-      int blocks = (int)((nb.size() + wpb - 1) / wpb);
-      eliminate_kernel<<<blocks, wpb * 32, in_smem ? per_warp * wpb : 0, s>>>(args);
+      const int wpb = S.nodes_per_block, blocks = (int)((nb.size() + wpb - 1) / wpb);
+      eliminate_kernel<<<blocks, wpb * 32, S.node_smem * wpb, s>>>(args);
       RCHOL_CUDA(cudaGetLastError());
-      if (!in_smem) RCHOL_CUDA(cudaStreamSynchronize(s));  // `wide` is freed on scope exit
+      if (!S.node_smem) RCHOL_CUDA(cudaStreamSynchronize(s));  // `wide` is freed on scope exit
     }
-    int hflags[NFLAGS];
-    flags.download(hflags, NFLAGS, s);
+    std::vector<int> hflags(nflags);
+    flags.download(hflags.data(), nflags, s);
     RCHOL_CUDA(cudaStreamSynchronize(s));
-    if (hflags[FLAG_FILL] || hflags[FLAG_WIDTH]) {
-      widest = std::max(widest, hflags[FLAG_WIDTH]);
+    const bool too_wide = std::any_of(hflags.begin() + NFLAGS, hflags.end(), [](int w) { return w > 0; });
+    if (hflags[FLAG_FILL] || too_wide) {
+      for (int d = 0; d <= maxdepth; ++d) widest[d] = std::max(widest[d], hflags[NFLAGS + d]);
       // Counts past an overflow are lower bounds (truncated columns sample
       // less fill into the columns after them).  Overflowing columns grow to
       // twice their count.  The other columns of an overflowing depth grow
