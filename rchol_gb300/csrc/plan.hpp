@@ -171,6 +171,7 @@ struct SegWork {
   uint64_t key_uid = 0;
   std::vector<int64_t> seg_host;
   int64_t n = 0;
+  bool one_block = false;  // short systems: a thread block per system makes its sums and updates
   DevBuf<int64_t> seg;
   DevBuf<double> r, z, p, q, x, sc;
   DevBuf<double> hb, hx;

@@ -1029,6 +1029,11 @@ __global__ void __launch_bounds__(SEG_THREADS) seg_init_kernel(SegState st, cons
 
 constexpr int SEG_GROUPS = SEG_THREADS / 32;  // warps of a system
 constexpr int SEG_AHEAD = 24;                 // rows of a chain read at a time
+// Longest system of the one-block kernels.  Whole solves, chains over eight
+// warps / one block: 50 systems of about 100 rows 834 / 622 us, 300 of 1024
+// 2.85 / 2.36 ms, 300 of 4096 7.27 / 7.17, 300 of 8100 12.8 / 13.4, one of
+// 4096 2.92 / 2.95, one of 16,384 10.0 / 11.3.
+constexpr int64_t kSegOneRows = 4096;
 
 // This warp's system (-1: none left, or converged) and chains.
 struct SegLane {
@@ -1133,17 +1138,63 @@ __global__ void __launch_bounds__(SEG_THREADS) seg_alpha_kernel(SegState st, con
   }
 }
 
-// The stopping test, one warp per system.
+// The stopping test of system s, ||r||^2 = rr; one thread.
+__device__ __forceinline__ void seg_stop(const SegState &st, int s, double rr) {
+  const int it = st.iters[s] + 1;
+  st.iters[s] = it;
+  st.rz_prev[s] = st.rz[s];
+  st.active[s] = (sqrt(rr) > sqrt(st.bnorm2[s]) * *st.tol) && (it < *st.maxit);
+}
+
+// One warp per system.
 __global__ void __launch_bounds__(128) seg_conv_kernel(SegState st) {
   const int s = (int)(blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32);
   if (s >= st.nseg || !*st.any_active || !st.active[s]) return;
   const double t = seg_total(seg_chains(st, 2, s));
-  if ((threadIdx.x & 31) == 0) {
-    const int it = st.iters[s] + 1;
-    st.iters[s] = it;
-    st.rz_prev[s] = st.rz[s];
-    st.active[s] = (sqrt(t) > sqrt(st.bnorm2[s]) * *st.tol) && (it < *st.maxit);
+  if ((threadIdx.x & 31) == 0) seg_stop(st, s, t);
+}
+
+// Short systems: one thread block per system makes a system's sums and updates
+// in one go, with two kernels an iteration instead of six.  (First of the two:
+// beta and p as above.)
+__global__ void __launch_bounds__(SEG_THREADS) seg_beta_one_kernel(SegState st, const double *r, const double *z,
+                                                                   double *p) {
+  __shared__ double sh[SEG_THREADS];
+  const int s = blockIdx.x;
+  if (!*st.any_active || !st.active[s]) return;
+  const int64_t i0 = st.seg[s], i1 = st.seg[s + 1];
+  double acc = 0.0;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += SEG_THREADS) acc += r[i] * z[i];
+  const double rz = seg_sum(acc, sh);
+  const int it = st.iters[s];
+  const double beta = it == 0 ? 0.0 : rz / st.rz_prev[s];
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += SEG_THREADS) p[i] = it == 0 ? z[i] : beta * p[i] + 1.0 * z[i];
+  if (threadIdx.x == 0) st.rz[s] = rz;
+}
+
+// Second: alpha, x and r as above, then the stopping test.
+__global__ void __launch_bounds__(SEG_THREADS) seg_alpha_one_kernel(SegState st, const double *p, const double *q,
+                                                                    double *x, double *r) {
+  __shared__ double sh[SEG_THREADS];
+  const int s = blockIdx.x;
+  if (!*st.any_active || !st.active[s]) return;
+  const int64_t i0 = st.seg[s], i1 = st.seg[s + 1];
+  double a0 = 0.0, a1 = 0.0;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += SEG_THREADS) {
+    const double pv = p[i];
+    a0 += pv * q[i];
+    a1 += pv * r[i];
   }
+  const double pq = seg_sum(a0, sh), pr = seg_sum(a1, sh), alpha = pr / pq;
+  double rr = 0.0;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += SEG_THREADS) {
+    x[i] += alpha * p[i];
+    const double rv = r[i] + -alpha * q[i];
+    r[i] = rv;
+    rr += rv * rv;
+  }
+  const double t = seg_sum(rr, sh);
+  if (threadIdx.x == 0) seg_stop(st, s, t);
 }
 
 __global__ void seg_any_kernel(SegState st) {
@@ -1173,6 +1224,13 @@ __global__ void __launch_bounds__(SEG_THREADS) seg_resid_kernel(SegState st, con
 
 }  // namespace
 
+// Whether a thread block per system serves (see the kernels).
+static bool seg_one_block(int64_t nseg, const int64_t *seg) {
+  int64_t most = 0;
+  for (int64_t s = 0; s < nseg; ++s) most = std::max(most, seg[s + 1] - seg[s]);
+  return most <= kSegOneRows;
+}
+
 static SegWork &seg_workspace(const rchol_matrix_s &A, const rchol_factor_s &F, int64_t nseg,
                               const int64_t *seg) {
   SolvePlan &P = *F.plan;
@@ -1191,7 +1249,8 @@ static SegWork &seg_workspace(const rchol_matrix_s &A, const rchol_factor_s &F, 
   w->p.alloc(A.n);
   w->q.alloc(A.n);
   w->x.alloc(A.n);
-  w->sc.alloc(4 * (size_t)nseg + 1 + 3 * (size_t)nseg * SEG_THREADS);
+  w->one_block = seg_one_block(nseg, seg);
+  w->sc.alloc(4 * (size_t)nseg + 1 + (w->one_block ? 0 : 3 * (size_t)nseg * SEG_THREADS));
   w->ic.alloc(2 * (size_t)nseg + 2);
   RCHOL_CUDA(cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking));
   RCHOL_CUDA(cudaEventCreateWithFlags(&w->ev_in, cudaEventDisableTiming));
@@ -1244,16 +1303,22 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
     RCHOL_CUDA(cudaStreamBeginCapture(ws, cudaStreamCaptureModeThreadLocal));
     try {
       precond_streams(F, w.r.p, w.z.p, 1, ws);
-      const unsigned C = S * SEG_GROUPS;
-      // element updates: enough parts of a system for four thread blocks an SM
-      const dim3 E(S, std::min(64u, (4 * seg_sms() + S - 1) / S));
-      seg_dot_kernel<false><<<C, 32, 0, ws>>>(st, 0, w.r.p, w.z.p, nullptr);
-      seg_beta_kernel<<<E, SEG_THREADS, 0, ws>>>(st, w.z.p, w.p.p);
-      spmv(A, w.p.p, w.q.p, 1, ws);
-      seg_dot_kernel<true><<<C, 32, 0, ws>>>(st, 0, w.p.p, w.q.p, w.r.p);
-      seg_alpha_kernel<<<E, SEG_THREADS, 0, ws>>>(st, w.p.p, w.q.p, w.x.p, w.r.p);
-      seg_dot_kernel<false><<<C, 32, 0, ws>>>(st, 2, w.r.p, w.r.p, nullptr);
-      seg_conv_kernel<<<(S + 3) / 4, 128, 0, ws>>>(st);
+      if (w.one_block) {
+        seg_beta_one_kernel<<<S, SEG_THREADS, 0, ws>>>(st, w.r.p, w.z.p, w.p.p);
+        spmv(A, w.p.p, w.q.p, 1, ws);
+        seg_alpha_one_kernel<<<S, SEG_THREADS, 0, ws>>>(st, w.p.p, w.q.p, w.x.p, w.r.p);
+      } else {
+        const unsigned C = S * SEG_GROUPS;
+        // element updates: enough parts of a system for four thread blocks an SM
+        const dim3 E(S, std::min(64u, (4 * seg_sms() + S - 1) / S));
+        seg_dot_kernel<false><<<C, 32, 0, ws>>>(st, 0, w.r.p, w.z.p, nullptr);
+        seg_beta_kernel<<<E, SEG_THREADS, 0, ws>>>(st, w.z.p, w.p.p);
+        spmv(A, w.p.p, w.q.p, 1, ws);
+        seg_dot_kernel<true><<<C, 32, 0, ws>>>(st, 0, w.p.p, w.q.p, w.r.p);
+        seg_alpha_kernel<<<E, SEG_THREADS, 0, ws>>>(st, w.p.p, w.q.p, w.x.p, w.r.p);
+        seg_dot_kernel<false><<<C, 32, 0, ws>>>(st, 2, w.r.p, w.r.p, nullptr);
+        seg_conv_kernel<<<(S + 3) / 4, 128, 0, ws>>>(st);
+      }
       seg_any_kernel<<<1, 256, 0, ws>>>(st);
       RCHOL_CUDA(cudaGetLastError());
     } catch (...) {
