@@ -44,82 +44,149 @@ __global__ void spmv1_kernel(int64_t n, const int64_t *__restrict__ rp, const in
   if (sub == 0 && row < n) y[row] = s;
 }
 
+// Up to W entries of a row (`on` of them are there) times V right-hand sides,
+// added in order.  All are read before the first is used.  W is the most that
+// any row of the warp has, so entries that no row has cost nothing: under a
+// condition the compiler keeps the multiply-add and selects, and at 2 of them
+// a clock and SM they are what a product with many right-hand sides waits for
+// (600^2 with 32: 156 us in rounds of 4 conditional entries).
+template <int V, int W>
+__device__ __forceinline__ void spmvk_add(double (&s)[V], const int32_t *__restrict__ ci, const double *__restrict__ v,
+                                          const double *__restrict__ x, int64_t row, int k, int on) {
+  double w[W], xv[W][V];
+#pragma unroll
+  for (int e = 0; e < W; ++e) {
+    const int64_t c = e < on ? ci[e] : row;
+    w[e] = e < on ? v[e] : 0.0;
+    if (V == 2) {
+      const double2 t = *reinterpret_cast<const double2 *>(x + c * k);
+      xv[e][0] = t.x, xv[e][V - 1] = t.y;
+    } else {
+      xv[e][0] = x[c * k];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < W; ++e)
+    if (e < on) {
+#pragma unroll
+      for (int u = 0; u < V; ++u) s[u] += w[e] * xv[e][u];
+    }
+}
+
 // y = A x for k right-hand sides stored row-major.  A thread owns V (1 or 2)
 // neighbouring right-hand sides of a row, k / V threads a row, so every load
 // of x and store of y is contiguous across a row's threads; the row's entries
-// are read four at a time and summed in order.  Bound by memory: 80^3
-// checkerboard, k = 8 (112 MB): 193 us with a warp per row (8 lanes of 32 at
-// work, one entry in flight), 61 us now,
-// near the 47 us that its 28.6 M FP64 multiply-adds take at 2 a clock and SM.
+// are read in rounds of up to eight and summed in order.  Bound by FP64
+// multiply-adds (2 a clock and SM): 80^3 with 8 takes 60 us, 47 of them for
+// its 28.6 M, and a warp per row 193; 600^2 with 2 11 us against 101.
 template <int V>
-__global__ void __launch_bounds__(256) spmvk_kernel(int64_t n, int k, const int64_t *__restrict__ rp,
+__global__ void __launch_bounds__(256) spmvk_kernel(int64_t n, int k, int rows, const int64_t *__restrict__ rp,
                                                     const int32_t *__restrict__ ci, const double *__restrict__ v,
                                                     const double *__restrict__ x, double *__restrict__ y) {
-  const int per_row = k / V, rows = 256 / per_row;  // of a thread block
-  const int lr = (int)threadIdx.x / per_row, r = ((int)threadIdx.x - lr * per_row) * V;
-  const int64_t row = blockIdx.x * (int64_t)rows + lr;
-  if (lr >= rows || row >= n) return;
-  const int64_t q1 = rp[row + 1];
+  const int per_row = k / V, lr = (int)threadIdx.x / per_row, r = ((int)threadIdx.x - lr * per_row) * V;
+  const int64_t row = min(blockIdx.x * (int64_t)rows + lr, n - 1);
+  const bool mine = lr < rows && blockIdx.x * (int64_t)rows + lr < n;
+  const int64_t q0 = rp[row];
+  const int len = mine ? (int)(rp[row + 1] - q0) : 0;
+  const int most = __reduce_max_sync(0xffffffffu, len);
+  ci += q0;
+  v += q0;
+  x += r;
   double s[V];
 #pragma unroll
   for (int u = 0; u < V; ++u) s[u] = 0.0;
-  for (int64_t q = rp[row]; q < q1; q += 4) {
-    double w[4], xv[4][V];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const bool on = q + e < q1;
-      const int64_t c = on ? ci[q + e] : row;
-      w[e] = on ? v[q + e] : 0.0;
-      if (V == 2) {
-        const double2 t = *reinterpret_cast<const double2 *>(x + c * k + r);
-        xv[e][0] = t.x, xv[e][V - 1] = t.y;
-      } else {
-        xv[e][0] = x[c * k + r];
-      }
+  for (int j = 0; j < most; j += 8, ci += 8, v += 8) switch (min(8, most - j)) {
+      case 1: spmvk_add<V, 1>(s, ci, v, x, row, k, len - j); break;
+      case 2: spmvk_add<V, 2>(s, ci, v, x, row, k, len - j); break;
+      case 3: spmvk_add<V, 3>(s, ci, v, x, row, k, len - j); break;
+      case 4: spmvk_add<V, 4>(s, ci, v, x, row, k, len - j); break;
+      case 5: spmvk_add<V, 5>(s, ci, v, x, row, k, len - j); break;
+      case 6: spmvk_add<V, 6>(s, ci, v, x, row, k, len - j); break;
+      case 7: spmvk_add<V, 7>(s, ci, v, x, row, k, len - j); break;
+      default: spmvk_add<V, 8>(s, ci, v, x, row, k, len - j);
     }
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (q + e < q1) {
-#pragma unroll
-        for (int u = 0; u < V; ++u) s[u] += w[e] * xv[e][u];
-      }
-  }
+  if (!mine) return;
   if (V == 2) *reinterpret_cast<double2 *>(y + row * k + r) = make_double2(s[0], s[V - 1]);
   else y[row * k + r] = s[0];
 }
 
+// Rows of a thread block with `per_row` threads each: as many as 256 threads
+// hold, fewer where that leaves over 5% of the last warp's round empty.
+int spmvk_rows(int per_row) {
+  auto fill = [per_row](int rows) { return (double)(rows * per_row) / ((rows * per_row + 31) / 32 * 32); };
+  int rows = 256 / per_row;
+  if (fill(rows) >= 0.95) return rows;
+  for (int t = rows - 1; t * per_row >= 128; --t)
+    if (fill(t) > fill(rows)) rows = t;
+  return rows;
+}
+
+// The same by one warp per row, lanes over the right-hand sides.
+__global__ void __launch_bounds__(256) spmvk_warp_kernel(int64_t n, int k, const int64_t *__restrict__ rp,
+                                                         const int32_t *__restrict__ ci, const double *__restrict__ v,
+                                                         const double *__restrict__ x, double *__restrict__ y) {
+  const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (row >= n) return;
+  for (int r = threadIdx.x & 31; r < k; r += 32) {
+    double s = 0.0;
+    for (int64_t q = rp[row]; q < rp[row + 1]; ++q) s += v[q] * x[(int64_t)ci[q] * k + r];
+    y[row * k + r] = s;
+  }
+}
+
+// Whether a warp per row serves k right-hand sides: where at least 7 of 8
+// lanes have one.  us, a warp per row / threads with pairs: 600^2 grid k = 26
+// 116 / 111, 28 117 / 117, 32 117 / 129, 48 201 / 172, 56 201 / 223, 64
+// 201 / 247; 60^3 k = 28 86 / 85, 32 86 / 94, 48 164 / 127, 64 164 / 176.
+bool spmvk_by_warps(int k) { return 8 * k >= 7 * ((k + 31) / 32 * 32); }
+
+// W entries of a slice's row, all read before the first gather; even ones to
+// s0, odd ones to s1.
+template <int W>
+__device__ __forceinline__ void sell_add(double &s0, double &s1, const int32_t *__restrict__ ci,
+                                         const double *__restrict__ v, const double *__restrict__ x) {
+  int32_t c[W];
+  double a[W], b[W];
+#pragma unroll
+  for (int u = 0; u < W; ++u) c[u] = __ldg(ci + 32 * u), a[u] = __ldg(v + 32 * u);
+#pragma unroll
+  for (int u = 0; u < W; ++u) b[u] = __ldg(&x[c[u]]);
+#pragma unroll
+  for (int u = 0; u < W; ++u) {
+    if (u & 1) s1 += a[u] * b[u];
+    else s0 += a[u] * b[u];
+  }
+}
+
 // y = A x, sliced ELL: one thread per row, each of a warp's loads is one
-// contiguous 128/256-byte transaction; eight entries are read, then gathered,
-// then added to two sums in turn.  Bound by HBM: 128^3 (226 MB) 49 us with two
-// entries in flight, 47.8 us now.
-__global__ void __launch_bounds__(256) spmv_sell_kernel(int64_t n, const int64_t *__restrict__ off,
-                                                        const int32_t *__restrict__ ci,
-                                                        const double *__restrict__ v,
-                                                        const double *__restrict__ x, double *__restrict__ y) {
+// contiguous 128/256-byte transaction.  A slice (a warp) reads its entries in
+// rounds of eight and a last one of just what is left (six thread blocks an SM
+// keep enough of them in flight).  Bound by HBM: 128^3 (226 MB) 39 us, 5.8
+// TB/s; with two entries in flight 49, with rounds of eight under conditions
+// and their 47 registers 48, where 2D grids, 5 of 8 entries, lost 20 to 40%
+// (300^2 4.5 -> 6.3 us, now 4.4).
+__global__ void __launch_bounds__(256, 6) spmv_sell_kernel(int64_t n, const int64_t *__restrict__ off,
+                                                           const int32_t *__restrict__ ci,
+                                                           const double *__restrict__ v,
+                                                           const double *__restrict__ x, double *__restrict__ y) {
   const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (row >= n) return;
   const int64_t sl = row >> 5;
   const int64_t o0 = off[sl];
-  const int w = (int)((off[sl + 1] - o0) >> 5);
+  int w = (int)((off[sl + 1] - o0) >> 5);
   ci += o0 + (row & 31);
   v += o0 + (row & 31);
   double s0 = 0.0, s1 = 0.0;
-  for (int j = 0; j < w; j += 8) {
-    int32_t c[8];
-    double a[8], b[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const bool on = j + u < w;
-      c[u] = on ? __ldg(ci + 32 * (j + u)) : (int32_t)row;
-      a[u] = on ? __ldg(v + 32 * (j + u)) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) b[u] = __ldg(&x[c[u]]);
-#pragma unroll
-    for (int u = 0; u < 8; u += 2) {
-      if (j + u < w) s0 += a[u] * b[u];
-      if (j + u + 1 < w) s1 += a[u + 1] * b[u + 1];
-    }
+  for (; w > 8; w -= 8, ci += 256, v += 256) sell_add<8>(s0, s1, ci, v, x);
+  switch (w) {
+    case 1: sell_add<1>(s0, s1, ci, v, x); break;
+    case 2: sell_add<2>(s0, s1, ci, v, x); break;
+    case 3: sell_add<3>(s0, s1, ci, v, x); break;
+    case 4: sell_add<4>(s0, s1, ci, v, x); break;
+    case 5: sell_add<5>(s0, s1, ci, v, x); break;
+    case 6: sell_add<6>(s0, s1, ci, v, x); break;
+    case 7: sell_add<7>(s0, s1, ci, v, x); break;
+    case 8: sell_add<8>(s0, s1, ci, v, x); break;
   }
   y[row] = s0 + s1;
 }
@@ -133,13 +200,16 @@ void spmv(const rchol_matrix_s &A, const double *x, double *y, int k, cudaStream
     int64_t threads = n * 8;
     spmv1_kernel<8><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(n, A.rp.p, A.ci.p, A.v.p, x, y);
     note_launch();
+  } else if (spmvk_by_warps(k)) {
+    spmvk_warp_kernel<<<(unsigned)((n * 32 + 255) / 256), 256, 0, s>>>(n, k, A.rp.p, A.ci.p, A.v.p, x, y);
+    note_launch();
   } else {
     // pairs of right-hand sides where every pair is 16-byte aligned
     const bool pairs = k % 2 == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0;
-    const int64_t rows = 256 / (pairs ? k / 2 : k);
-    const unsigned grid = (unsigned)((n + rows - 1) / rows);
-    if (pairs) spmvk_kernel<2><<<grid, 256, 0, s>>>(n, k, A.rp.p, A.ci.p, A.v.p, x, y);
-    else spmvk_kernel<1><<<grid, 256, 0, s>>>(n, k, A.rp.p, A.ci.p, A.v.p, x, y);
+    const int per_row = pairs ? k / 2 : k, rows = spmvk_rows(per_row);
+    const unsigned grid = (unsigned)((n + rows - 1) / rows), threads = (unsigned)(rows * per_row + 31) / 32 * 32;
+    if (pairs) spmvk_kernel<2><<<grid, threads, 0, s>>>(n, k, rows, A.rp.p, A.ci.p, A.v.p, x, y);
+    else spmvk_kernel<1><<<grid, threads, 0, s>>>(n, k, rows, A.rp.p, A.ci.p, A.v.p, x, y);
     note_launch();
   }
   RCHOL_CUDA(cudaGetLastError());
