@@ -20,9 +20,9 @@ from ._lib import PREC_FP32, Factor, Matrix, Tree
 
 def autotune_threads(mats, candidates=(1, 2, 4, 8, 16), sample=8, seed=0, precision=PREC_FP32, reps=3):
     """Leaves per system (the ``threads`` of Batch) chosen by measurement: the
-    largest ``sample`` systems are factored with every candidate and the
-    preconditioner apply (the dominant cost of a PCG iteration) is timed on
-    the GPU with CUDA events; the fastest candidate wins.  Returns
+    largest ``sample`` systems are factored with every candidate and solved by
+    batched PCG, as Batch.solve does, to its default tolerance; the candidate
+    whose solve takes the least time on the GPU (CUDA events) wins.  Returns
     (best, {candidate: ms})."""
     import torch
 
@@ -36,19 +36,22 @@ def autotune_threads(mats, candidates=(1, 2, 4, 8, 16), sample=8, seed=0, precis
             continue
         b = Batch(probe, threads=t, seed=seed, precision=precision)
         n = int(b.sys_ptr[-1])
-        d_r = torch.as_tensor(np.random.default_rng(seed).standard_normal(n), device="cuda")
-        d_z = torch.empty_like(d_r)
+        d_b = torch.as_tensor(np.random.default_rng(seed).standard_normal(n), device="cuda")
+        d_x = torch.empty_like(d_b)
+        relres = np.zeros(b.nsys)
+        itr = np.zeros(b.nsys, dtype=np.int32)
 
-        def apply():
-            _lib.check(_lib.lib().rchol_gpu_precond_d(b.F.ptr, d_r.data_ptr(), d_z.data_ptr(), 1,
-                                                      stream.cuda_stream))
+        def solve():
+            _lib.check(_lib.lib().rchol_gpu_pcg_batch_d(b.A.ptr, b.F.ptr, b.nsys, _lib.p64(b.sys_ptr), d_b.data_ptr(),
+                                                        d_x.data_ptr(), 1e-8, 200, _lib.pd(relres),
+                                                        itr.ctypes.data_as(_lib._ip), stream.cuda_stream))
 
-        apply()
+        solve()
         e0 = torch.cuda.Event(enable_timing=True)
         e1 = torch.cuda.Event(enable_timing=True)
         e0.record(stream)
         for _ in range(reps):
-            apply()
+            solve()
         e1.record(stream)
         torch.cuda.synchronize()
         timings[t] = e0.elapsed_time(e1) / reps
