@@ -480,6 +480,19 @@ __device__ __forceinline__ uint2 lds8(uint32_t a) {
 __device__ __forceinline__ void lds_val(uint32_t a, float &v) { asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(v) : "r"(a) : "memory"); }
 __device__ __forceinline__ void lds_val(uint32_t a, double &v) { asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v) : "r"(a) : "memory"); }
 
+// Whether any of four sums is a NaN or an infinity (FP32: or their sum, which
+// is as good; FP64 additions are scarce).
+__device__ __forceinline__ bool not_finite(const float (&x)[4]) {
+  return (__float_as_uint((x[0] + x[1]) + (x[2] + x[3])) & 0x7f800000u) == 0x7f800000u;
+}
+__device__ __forceinline__ bool not_finite(const double (&x)[4]) {
+  bool any = false;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) any |= (__double2hiint(x[r]) & 0x7ff00000) == 0x7ff00000;
+  return any;
+}
+
+// 16 bytes of values; dot_nonzero leaves out the terms where this one is zero.
 template <typename VT>
 struct Vec16;
 template <>
@@ -492,6 +505,13 @@ struct Vec16<float> {
   __device__ __forceinline__ float dot(const Vec16 &b, float s) const {
     return fmaf(v.w, b.v.w, fmaf(v.z, b.v.z, fmaf(v.y, b.v.y, fmaf(v.x, b.v.x, s))));
   }
+  __device__ __forceinline__ float dot_nonzero(const Vec16 &b, float s) const {
+    if (v.x != 0.f) s = fmaf(v.x, b.v.x, s);
+    if (v.y != 0.f) s = fmaf(v.y, b.v.y, s);
+    if (v.z != 0.f) s = fmaf(v.z, b.v.z, s);
+    if (v.w != 0.f) s = fmaf(v.w, b.v.w, s);
+    return s;
+  }
 };
 template <>
 struct Vec16<double> {
@@ -502,6 +522,11 @@ struct Vec16<double> {
   __device__ __forceinline__ double get(int i) const { return i & 1 ? v.y : v.x; }
   __device__ __forceinline__ double dot(const Vec16 &b, double s) const {
     return fma(v.y, b.v.y, fma(v.x, b.v.x, s));
+  }
+  __device__ __forceinline__ double dot_nonzero(const Vec16 &b, double s) const {
+    if (v.x != 0.0) s = fma(v.x, b.v.x, s);
+    if (v.y != 0.0) s = fma(v.y, b.v.y, s);
+    return s;
   }
 };
 
@@ -580,8 +605,21 @@ __device__ __forceinline__ VT ext_sum(uint32_t cols, uint32_t vals, uint32_t q, 
 // The thread after the row threads streams the records: record s+2 is waited
 // for in step s.  One block-wide barrier per step, which also carries a
 // failed wait.
+// Registers: where many thread blocks share an SM, the compiler's choice would
+// leave out one of them.  FP32 with one vector of the inverse per row is held
+// to 64 (it would take 83 for the branch on infinities: 12^3 with 32 columns
+// 52 -> 65 us), with two in a cluster to 80 (104: 64^3 with 32 columns 1.42 ->
+// 1.49 ms; 64: with one column 246 -> 320 us).  A launch has 384 threads at
+// most: 256 row threads and 128 helpers.
+template <typename VT, int NV, bool CLUSTER>
+struct BlkBounds {
+  static constexpr bool pairs = NV == 2 && CLUSTER && sizeof(VT) == 4;
+  static constexpr int threads = pairs ? 384 : 512;
+  static constexpr int blocks = pairs || (NV == 1 && (CLUSTER || sizeof(VT) == 4)) ? 2 : 1;
+};
 template <typename VT, typename InT, typename OutT, bool UPPER, int NV, bool CLUSTER>
-__global__ void __launch_bounds__(512) blk_solve_kernel(BlkArgs<VT> a, const InT *in, OutT *out) {
+__global__ void __launch_bounds__(BlkBounds<VT, NV, CLUSTER>::threads, BlkBounds<VT, NV, CLUSTER>::blocks)
+    blk_solve_kernel(BlkArgs<VT> a, const InT *in, OutT *out) {
   allow_next();
   extern __shared__ __align__(16) unsigned char smem[];
   const int C = CLUSTER ? a.C : 1;
@@ -799,6 +837,16 @@ __global__ void __launch_bounds__(512) blk_solve_kernel(BlkArgs<VT> a, const InT
 #pragma unroll
           for (int r = 0; r < 4; ++r) x[r] = m[v][r].dot(tv[v], x[r]);
         }
+      if (not_finite(x)) {
+        // A NaN or an infinity in t: the inverse's zeros must not carry it to
+        // rows that do not depend on it.
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          x[r] = VT(0);
+#pragma unroll
+          for (int v = 0; v < NV; ++v) x[r] = m[v][r].dot_nonzero(tv[v], x[r]);
+        }
+      }
       {  // fold: after two exchanges each quarter of the group holds its own row
         const bool hi = lg & (GL >> 1), hi2 = lg & (GL >> 2);
         const VT y0 = hi ? x[2] : x[0], y1 = hi ? x[3] : x[1];
