@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(BlkBounds<VT, NV, CLUSTER>::threads, BlkBounds
     for (int s = 0; s < nb; ++s) {
       if (CLUSTER && s > 0) {
         if (!dead && !mbar_wait(xbar, (uint32_t)(s - 1) & 1u)) give_up();
-        if (tid == 0) mbar_expect(xbar, block_bytes(s));
+        if (tid == 0 && !dead) mbar_expect(xbar, block_bytes(s));  // one arrival per phase
       }
       stop = __syncthreads_or(dead) || stop;
       VT sum = part;
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(BlkBounds<VT, NV, CLUSTER>::threads, BlkBounds
         send(t_dst, t_bar, left > 0 ? ps[(s & 1) * nown + j] - sum : VT(0));
         if (!stop && s + 1 < nb) open_record();
         if (!dead && !mbar_wait(tbar, (uint32_t)s & 1u)) give_up();
-        if (tid == 0 && s + 1 < nb) mbar_expect(tbar, block_bytes(s + 1));
+        if (tid == 0 && !dead && s + 1 < nb) mbar_expect(tbar, block_bytes(s + 1));
         __syncwarp();
       } else {
         if (l == 0) tb[pos] = left > 0 ? rhs - sum : VT(0);
@@ -903,8 +903,11 @@ __global__ void __launch_bounds__(BlkBounds<VT, NV, CLUSTER>::threads, BlkBounds
     }
   }
   if (CLUSTER) {
-    if (!dead) (void)mbar_wait(xbar, (uint32_t)(nb - 1) & 1u);
+    if (!dead && !mbar_wait(xbar, (uint32_t)(nb - 1) & 1u)) give_up();
     cluster_sync();  // nobody leaves while others may still send here
+    // Without a completed phase the others' last stores, all issued by now, may
+    // still be on their way: they take microseconds.
+    if (dead) __nanosleep(1000000);
   }
 }
 
