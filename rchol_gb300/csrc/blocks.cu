@@ -24,6 +24,7 @@
 // distance, lay out the records, copy the entries, invert the triangles.
 
 #include <algorithm>
+#include <array>
 #include <cstring>
 #include <mutex>
 
@@ -917,6 +918,8 @@ __global__ void __launch_bounds__(BlkBounds<VT, NV, CLUSTER>::threads, BlkBounds
 
 namespace {
 
+using ClusterFit = std::array<int, 5>;
+
 // Cluster size, block rows and threads of a stage of npieces pieces, the
 // longest with maxrows rows.
 //
@@ -933,9 +936,12 @@ namespace {
 // In FP64 (2 FMA per clock and SM) the inverse's B / 2 products per row are
 // what a step costs, so B is smaller: 417 us for 64^3 with 64 subdomains
 // against 451 with B = 128 at the root and 1066 with the record streams.
-void choose_shape(BlkStage &S, bool fp32, int cols) {
+// fit: clusters of 1, 2, 4, 8, 16 that the device runs at once; a size that it
+// does not run at all gives way to the next smaller one.
+void choose_shape(BlkStage &S, bool fp32, int cols, const ClusterFit &fit) {
   const int P = (int)std::min<int64_t>((int64_t)S.npieces * cols, 1 << 20), R = S.maxrows;
-  const int i = P <= 8 && R >= 512 ? 4 : P <= 18 && R >= 256 ? 3 : P <= 36 && R >= 128 ? 2 : P <= 76 && R >= 128 ? 1 : 0;
+  int i = P <= 8 && R >= 512 ? 4 : P <= 18 && R >= 256 ? 3 : P <= 36 && R >= 128 ? 2 : P <= 76 && R >= 128 ? 1 : 0;
+  while (i > 0 && fit[i] < 1) --i;
   static const int b32[] = {64, 128, 256, 256, 512}, b64[] = {32, 64, 128, 128, 256};
   static const int g32[] = {8, 16, 16, 32, 32}, g64[] = {16, 16, 32, 32, 32};
   S.C = 1 << i;
@@ -965,6 +971,41 @@ void set_geometry(BlkStage &S, size_t vsz) {
   S.stride = (int64_t)S.goff[nown / 4] * per;
 }
 
+constexpr int kMaxDevices = 128;
+
+// Clusters of 1, 2, 4, 8 and 16 thread blocks, one per SM, that run at once on
+// the current device (152, 76, 36, 15 and 7 on a whole GB300); asked once.
+const ClusterFit &cluster_fit() {
+  static std::once_flag once[kMaxDevices];
+  static ClusterFit fit[kMaxDevices];
+  int dev = 0;
+  RCHOL_CUDA(cudaGetDevice(&dev));
+  RCHOL_CHECK_ARG(dev >= 0 && dev < kMaxDevices, "device ordinal out of range");
+  std::call_once(once[dev], [&] {
+    auto *kernel = blk_solve_kernel<float, float, double, true, 1, true>;
+    RCHOL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlkSmem));
+    RCHOL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    RCHOL_CUDA(cudaDeviceGetAttribute(&fit[dev][0], cudaDevAttrMultiProcessorCount, dev));
+    for (int i = 1; i < 5; ++i) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1u << i);
+      cfg.blockDim = dim3(256);
+      cfg.dynamicSmemBytes = kBlkSmem;
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = 1u << i;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&fit[dev][i], kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        fit[dev][i] = 0;
+      }
+    }
+  });
+  return fit[dev];
+}
+
 size_t stage_smem(const BlkStage &S, size_t vsz, int ring) {
   return kBlkBars + vsz * (size_t)(S.B + 2 * (S.B / S.C) + (S.maxrows + 3) / 4 * 4 + 4) + (size_t)ring * S.slot;
 }
@@ -972,6 +1013,7 @@ size_t stage_smem(const BlkStage &S, size_t vsz, int ring) {
 template <typename VT>
 bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, const DevBuf<double> &v,
                const std::vector<TreeNode> &tnodes, bool upper, int cols, BlkDir &D, DevBuf<VT> &inv, cudaStream_t s) {
+  const ClusterFit &fit = cluster_fit();
   int maxdepth = 1;
   for (auto &nd : tnodes) maxdepth = std::max(maxdepth, nd.depth);
   std::vector<BlkPiece> pieces;
@@ -998,7 +1040,7 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
       }
       S.npieces = (int)pieces.size() - S.piece0;
       if (!S.npieces) break;
-      choose_shape(S, sizeof(VT) == 4, cols);
+      choose_shape(S, sizeof(VT) == 4, cols, fit);
       D.stages.push_back(S);
     }
   }
@@ -1157,8 +1199,6 @@ bool build_dir(int64_t n, const DevBuf<int64_t> &rp, const DevBuf<int32_t> &ci, 
   return false;
 }
 
-constexpr int kMaxDevices = 128;
-
 // Launch of a kernel that calls wait_previous, in clusters of C thread blocks;
 // early: it may start before the kernel ahead of it has ended.
 template <typename... Params, typename... Args>
@@ -1205,8 +1245,7 @@ void launch_stage(const BlkStage &S, const BlkArgs<VT> &a, const InT *in, OutT *
   // 700^2 728, 1007, 644; 12^3 72, 47, 48.  FP64 stages of more than one wave
   // start in turn: they run long, and early ones were up to 4% slower (700^2
   // with 5 columns 1534 -> 1594 us).
-  const int side[] = {152, 76, 36, 15, 7};  // clusters of 1, 2, 4, 8, 16 that fit, one thread block per SM
-  const int fit = side[S.C == 1 ? 0 : S.C == 2 ? 1 : S.C == 4 ? 2 : S.C == 8 ? 3 : 4];
+  const int fit = std::max(1, cluster_fit()[S.C == 1 ? 0 : S.C == 2 ? 1 : S.C == 4 ? 2 : S.C == 8 ? 3 : 4]);
   const int64_t waves = ((int64_t)S.npieces * a.k + fit - 1) / fit;
   const bool early = sizeof(VT) == 4 || waves == 1;
   size_t smem = S.smem;
