@@ -1890,8 +1890,9 @@ static void build_dir_streams(const std::vector<int64_t> &rp, const std::vector<
   const int64_t nruns = (int64_t)built.size();
   std::vector<int32_t> chunks(nruns, 0);
   // one run at a time per thread, from the top of the tree with its long rows
+  // (no more threads than runs: to start 16 for one run took a millisecond)
   std::atomic<int64_t> next_run{0};
-  parallel_for(host_threads(), [&](int64_t, int64_t) {
+  parallel_for(std::min<int64_t>(host_threads(), nruns), [&](int64_t, int64_t) {
     for (int64_t i; (i = next_run.fetch_add(1)) < nruns;) {
       const int64_t r = upper ? i : nruns - 1 - i;
       const Piece &pc = pieces[run_piece[r]];
@@ -1935,7 +1936,7 @@ static void build_dir_streams(const std::vector<int64_t> &rp, const std::vector<
   std::unique_ptr<unsigned char[]> all(new unsigned char[std::max<int64_t>(total, 1)]);
   parallel_for(nruns, [&](int64_t r0, int64_t r1) {
     for (int64_t r = r0; r < r1; ++r) std::memcpy(all.get() + run_off[r], built[r].bytes.data(), built[r].bytes.size());
-  }, 1);
+  }, total < (1 << 20) ? nruns : 1);
   built.clear();
   // stages
   D.stage_rows.clear();
