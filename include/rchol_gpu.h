@@ -136,11 +136,12 @@ int rchol_gpu_factor_pivots(rchol_factor_t G, double *d);
  * pieces, and the sequential 32-row block steps on the critical path.  No
  * counterpart in the reference. */
 int rchol_gpu_factor_plan_info(rchol_factor_t G, int transpose, int64_t *stages, int64_t *pieces, int64_t *steps);
-/* Whether rchol_gpu_trsv_d and rchol_gpu_precond_d solve in large blocks (1)
- * or by the plan that PCG applies (0): G with an off-diagonal entry above
- * zero, with rows too dense, or with a block plan of over an eighth of the
- * device's memory per direction.  -1 without a factor.  No counterpart in the
- * reference. */
+/* Which plan rchol_gpu_trsv_d and rchol_gpu_precond_d take: 0 the one that PCG
+ * applies (G with an off-diagonal entry above zero, with rows too dense, or
+ * with a block plan of over an eighth of the device's memory per direction);
+ * 1 large blocks for several right-hand sides (many short independent
+ * systems); 2 large blocks always.  -1 without a factor.  No counterpart in
+ * the reference. */
 int rchol_gpu_factor_blocked(rchol_factor_t G);
 /* Autotuning of the preconditioner that PCG applies with this factor: times it
  * with alternative launch choices (L2 prefetch distance and ring depth of the

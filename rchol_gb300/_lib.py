@@ -262,9 +262,9 @@ class Factor(Handle):
         check(lib().rchol_gpu_factor_plan_info(self.ptr, int(transpose), C.byref(a), C.byref(b), C.byref(c)))
         return a.value, b.value, c.value
 
-    def blocked(self):
-        """Whether trsv and precond solve in large blocks."""
-        return bool(lib().rchol_gpu_factor_blocked(self.ptr))
+    def blocked(self, k=1):
+        """Whether trsv and precond with k right-hand sides solve in large blocks."""
+        return lib().rchol_gpu_factor_blocked(self.ptr) >= (2 if k == 1 else 1)
 
     def tune(self):
         """Times the solves with alternative launch choices on this factor and

@@ -1370,6 +1370,27 @@ BlkBuilt build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s) {
   return try_build(P.bfwd, P.bbwd, [&] { return block_signs(F, s) && build_block_dirs(F, 1, P.bfwd, P.bbwd, s); });
 }
 
+// Whether one right-hand side is solved on the block plan, too (several always
+// are).  Its clusters shorten the chain of stages with few pieces; where a
+// stage's pieces take more than three rounds of all SMs, a warp per piece
+// (w2_kernel) gets more done than a thread block per piece.  us per
+// preconditioner, record streams / blocks: 400 systems of 512 rows FP32 33 /
+// 19, FP64 95 / 87; 500 of 1024 FP32 60 / 73, FP64 185 / 257; 3000 of 256 FP32
+// 55 / 90, FP64 199 / 267; 1000^2 grid with 4096 subdomains of 244 rows FP32 508
+// / 302, FP64 1142 / 693.  The figures below are least-squares lines through 170
+// such batches with 1 to 8 subdomains per system and single chains.
+bool blocks_for_one(const rchol_factor_s &F, const SolvePlan &P) {
+  const bool fp32 = F.precision == RCHOL_PREC_FP32;
+  const int rounds = 3 * cluster_fit()[0];
+  double gain = 0.0;  // us
+  for (const BlkStage &S : P.bfwd.stages) {
+    if (S.npieces <= rounds) gain += fp32 ? 9.0 + 0.028 * S.maxrows : 12.0 + 0.106 * S.maxrows;
+    else if (fp32) gain += 10.0 - 1e-3 * (8.0 * S.npieces + 0.03 * (double)S.rows);
+    else gain -= 1e-3 * (6.0 * S.npieces + 0.08 * (double)S.rows);
+  }
+  return gain >= 0.0;
+}
+
 void build_blocks_k(const rchol_factor_s &F, SolvePlan &P, int k, cudaStream_t s) {
   if (P.kblocks || k < kBlkWideFrom) return;
   P.kwide = try_build(P.bkfwd, P.bkbwd, [&] { return build_block_dirs(F, kBlkWideCols, P.bkfwd, P.bkbwd, s); }) ==

@@ -271,7 +271,9 @@ int rchol_gpu_factor_plan_info(rchol_factor_t G, int transpose, int64_t *stages,
   API_END
 }
 
-int rchol_gpu_factor_blocked(rchol_factor_t G) { return G && G->plan ? (int)G->plan->blocked : -1; }
+int rchol_gpu_factor_blocked(rchol_factor_t G) {
+  return G && G->plan ? (int)G->plan->blocked + (int)G->plan->blocked1 : -1;
+}
 
 int rchol_gpu_factor_tune(rchol_factor_t G, double *ms_before, double *ms_after, int *knobs) {
   API_BEGIN

@@ -206,6 +206,7 @@ struct SolvePlan {
   std::vector<std::unique_ptr<SegWork>> seg;
   unsigned int *status = nullptr;  // status word of the solve kernels
   bool blocked = false;    // trsv and precond run on bfwd / bbwd (else, and in PCG, on the record streams)
+  bool blocked1 = false;   // the same for one right-hand side
   BlkDir bfwd, bbwd;
   BlkDir bkfwd, bkbwd;     // shapes for several right-hand sides (built on first use)
   bool kblocks = false, kwide = false;  // that was tried; it is there
@@ -226,6 +227,8 @@ struct SolvePlan {
 // entries have mixed signs, or it would be too large.
 enum class BlkBuilt { kReady, kLeftOut, kNoMemory };
 BlkBuilt build_blocks(const rchol_factor_s &F, SolvePlan &P, cudaStream_t s);
+// Whether one right-hand side takes that plan.
+bool blocks_for_one(const rchol_factor_s &F, const SolvePlan &P);
 // The plan that k right-hand sides take, where it is another one.
 void build_blocks_k(const rchol_factor_s &F, SolvePlan &P, int k, cudaStream_t s);
 // Solve with G (upper = false) or G^T for k <= kBlkCols right-hand sides, one

@@ -558,6 +558,7 @@ void build_plan(rchol_factor_s &F, cudaStream_t s) {
     }
     if (built == BlkBuilt::kNoMemory) built = build_blocks(F, *P, s);
     P->blocked = built == BlkBuilt::kReady;
+    P->blocked1 = P->blocked && blocks_for_one(F, *P);
   } catch (...) {
     delete P;
     throw;
@@ -716,17 +717,18 @@ void trsv(const rchol_factor_s &F, bool upper, const double *in, double *out, in
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
-  if (P.blocked) ensure_blocks(F, k, s);
+  const bool blocks = k == 1 ? P.blocked1 : P.blocked;
+  if (blocks) ensure_blocks(F, k, s);
   else ensure_streams(F, k, s);
-  if (k == 1) trsv_one(F, P, P.blocked, upper, in, nullptr, out, nullptr, ensure_acc(P, fp32, F.n), s);
-  else if (P.blocked) blocks_k(F, P, upper, in, out, k, s);
+  if (k == 1) trsv_one(F, P, blocks, upper, in, nullptr, out, nullptr, ensure_acc(P, fp32, F.n), s);
+  else if (blocks) blocks_k(F, P, upper, in, out, k, s);
   else stream_trsv_k(F, P, upper, in, nullptr, out, nullptr, k, s);
 }
 
 void precond(const rchol_factor_s &F, const double *r, double *z, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
-  if (!P.blocked) {
+  if (!(k == 1 ? P.blocked1 : P.blocked)) {
     ensure_streams(F, k, s);
     precond_streams(F, r, z, k, s);
     return;
@@ -796,8 +798,8 @@ void precond_noalloc(const rchol_factor_s &F, const double *r, double *z, cudaSt
                                        std::to_string(kNoAllocScratchBytes / (2 * vsz)) + " for this precision)");
   unsigned char *base = static_cast<unsigned char *>(noalloc_scratch_address(s));
   void *y = base + acc_bytes;
-  precond_one(F, *F.plan, F.plan->blocked, r, z, fp32 ? nullptr : static_cast<double *>(y), fp32 ? static_cast<float *>(y) : nullptr,
-              base, s);
+  precond_one(F, *F.plan, F.plan->blocked1, r, z, fp32 ? nullptr : static_cast<double *>(y),
+              fp32 ? static_cast<float *>(y) : nullptr, base, s);
 }
 
 void spmv_public(const rchol_matrix_s &A, const double *x, double *y, int k, cudaStream_t s) {

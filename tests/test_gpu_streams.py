@@ -128,3 +128,27 @@ def test_which_factors_are_blocked(cuda, R, precision):
     w = v.copy()
     w[rp[100] + 1] = 0.0
     assert R.Factor.from_host(rp, ci, w, precision=precision).blocked()
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
+def test_many_short_systems(cuda, R, precision):
+    """One right-hand side of many short systems stays on the record streams
+    (a warp per system), several take the block plan; a tree with long
+    separators over as many subdomains takes it for one, too."""
+    import torch
+
+    A = generators.grid_2d_weighted(16, 16, "lognormal", sigma=0.5)
+    B = R.Batch([A] * 1000, threads=1, precision=precision)
+    assert not B.F.blocked(1) and B.F.blocked(2)
+    rp, ci, v = B.F.export()
+    U = sp.csr_matrix((v, ci, rp))
+    b = np.random.default_rng(1).standard_normal((U.shape[0], 2))
+    y = spl.spsolve_triangular(U.T.tocsr(), b, lower=True)
+    z = spl.spsolve_triangular(U, y, lower=False)
+    for k in (1, 2):
+        x = _apply(torch, B.F, 2, np.ascontiguousarray(b[:, :k]))
+        assert np.linalg.norm(x - z[:, :k]) <= 2 * TOL[precision] * np.linalg.norm(z[:, :k])
+    A = generators.laplace_3d(32)
+    tree = R.Tree.build(A.indptr, A.indices, 1024)
+    Ad = R.Matrix.create(A.indptr, A.indices, A.data, tree)
+    assert R.Factor.compute(Ad, tree, precision=precision).blocked(1)
