@@ -1334,7 +1334,6 @@ BlkBuilt try_build(BlkDir &fwd, BlkDir &bwd, Make make) {
     if (make()) return BlkBuilt::kReady;
   } catch (const Error &e) {
     if (e.status != RCHOL_ERR_NOMEM) throw;
-    (void)cudaGetLastError();  // the failed allocation's
     built = BlkBuilt::kNoMemory;
   }
   fwd = BlkDir();

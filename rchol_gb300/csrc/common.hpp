@@ -24,12 +24,16 @@ void set_last_error(const std::string &msg);
 // Counts kernel launches made by the solve path (rchol_gpu_launch_count).
 void note_launch(int64_t count = 1);
 
+// The error is thrown and taken out of the runtime: one left there (an
+// allocation that failed) would fail the next call's check of its launches.
 #define RCHOL_CUDA(call)                                                                  \
   do {                                                                                    \
     cudaError_t e_ = (call);                                                              \
-    if (e_ != cudaSuccess)                                                                \
+    if (e_ != cudaSuccess) {                                                              \
+      (void)cudaGetLastError();                                                           \
       throw ::rchol::Error(e_ == cudaErrorMemoryAllocation ? RCHOL_ERR_NOMEM : RCHOL_ERR_CUDA, \
                            std::string(#call) + ": " + cudaGetErrorString(e_));          \
+    }                                                                                     \
   } while (0)
 
 #define RCHOL_CHECK_ARG(cond, msg)                              \

@@ -547,7 +547,6 @@ void build_plan(rchol_factor_s &F, cudaStream_t s) {
       if (wanted) built = other.get();
     } catch (const Error &e) {
       if (!wanted || e.status != RCHOL_ERR_NOMEM) throw;
-      (void)cudaGetLastError();
       if (other.valid()) other.wait();
       P->bfwd = BlkDir();
       P->bbwd = BlkDir();

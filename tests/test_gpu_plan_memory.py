@@ -92,3 +92,21 @@ def test_factor_is_made_where_the_streams_fit(R, problem, monkeypatch, precision
         if not fits[True]:
             break
     assert made[True] and made[False]
+
+
+def test_call_after_one_without_memory(R, problem):
+    """A factor that could not be made leaves nothing behind that fails the
+    next call."""
+    import torch
+
+    tree, Ad, b = problem
+    filler = _fill(torch, 32 * MB)
+    try:
+        with pytest.raises(R.RcholError) as e:
+            R.Factor.compute(Ad, tree, seed=1)
+        assert e.value.status == _lib.ERR_NOMEM
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    F = R.Factor.compute(Ad, tree, seed=1)
+    assert bool(_solve(torch, F, b).isfinite().all())
