@@ -67,8 +67,8 @@ struct DevBuf {
   ~DevBuf() { release(); }
   void alloc(size_t count) {
     release();
-    n = count;
     if (count) RCHOL_CUDA(cudaMalloc(&p, count * sizeof(T)));
+    n = count;  // only now: users ask n whether they have to allocate
   }
   void release() {
     if (p) cudaFree(p);
