@@ -188,7 +188,10 @@ int rchol_gpu_pcg_batch(rchol_matrix_t A, rchol_factor_t G, int64_t nsys, const 
 int rchol_gpu_pcg_batch_d(rchol_matrix_t A, rchol_factor_t G, int64_t nsys,
                           const int64_t *sys_ptr, const double *d_b, double *d_x, double tol,
                           int maxit, double *relres, int *itr, void *stream);
-/* z = (G G^T)^-1 r (c++/util/pcg.cpp:141-159); device pointers. */
+/* z = (G G^T)^-1 r (c++/util/pcg.cpp:141-159); device pointers.  Where
+ * rchol_gpu_factor_blocked says so the solves run in large blocks, whose sums
+ * have another order than those inside PCG: both are as accurate, their last
+ * digits differ. */
 int rchol_gpu_precond_d(rchol_factor_t G, const double *d_r, double *d_z, int64_t nrhs,
                         void *stream);
 /* z = (G G^T)^-1 r for one right-hand side without allocating any memory.

@@ -1,4 +1,5 @@
-// Triangular solves with G and G^T in large blocks.
+// Triangular solves with G and G^T in large blocks: rchol_gpu_trsv_d and
+// rchol_gpu_precond_d (PCG applies the record streams of trsv.cu).
 //
 // Replaces the two MKL trsv calls of c++/util/pcg.cpp:141-159.
 //
@@ -18,7 +19,7 @@
 // column of a piece: the chain's length, not the arithmetic, is what a solve
 // costs, and columns hide it from one another.  Preconditioner of 80^3 with
 // 128 subdomains, record streams -> now: FP32 2 columns 8.9 -> 0.65 ms, 32
-// columns 8.3 -> 2.6; FP64 49 -> 1.5 and 49 -> 8.8 ms.
+// columns 8.3 -> 2.5; FP64 49 -> 1.5 and 49 -> 8.8 ms.
 //
 // The plan is built on the GPU from the CSR of G (or G^T): count entries by
 // distance, lay out the records, copy the entries, invert the triangles.
@@ -590,7 +591,7 @@ __device__ __forceinline__ VT ext_sum(uint32_t cols, uint32_t vals, uint32_t q, 
 // (product) and the shuffles of two sums.  Measured at 128^3 (FP32 forward,
 // the root's 16,384 rows, 32 steps of 512 by 16 thread blocks): 48 us, against
 // 293 us for 512 steps of 32 rows by one thread block (pipe_kernel); all
-// stages 507 us in turn, 455 us with early starts, against 1122 us.  The subdomains (512 pieces, 92% of the
+// stages 507 us in turn, 447 us with early starts, against 1122 us.  The subdomains (512 pieces, 92% of the
 // rows) take 132 us of it for 490 MB, 3.7 TB/s (w2_kernel: 200 us).
 //   row threads: gl lanes per group of four own rows, a quarter of them per
 //     row for the sparse sums.  Step s adds the row's entries in block s-1 to
