@@ -135,10 +135,10 @@ struct BlkDir {
   int64_t early_rows = 0;
 };
 
-// Vectors of solves on the block plan with up to `cols` right-hand sides:
-// right-hand sides and solutions column after column (cols > 1), and what lies
-// between the two solves of the preconditioner.
-struct BlkWork {
+// Vectors of trsv and precond with up to `cols` right-hand sides: what lies
+// between the two solves of the preconditioner, and on the block plan with
+// several of them right-hand sides and solutions column after column.
+struct SolveWork {
   int cols = 0;
   DevBuf<double> a, b, y64;
   DevBuf<float> y32;
@@ -214,13 +214,13 @@ struct SolvePlan {
   StreamDir kfwd, kbwd;    // pieces for up to 32 right-hand sides (built on first use)
   bool kbuilt = false;
   int64_t dag_fwd = -1, dag_bwd = -1;  // dependency-chain lengths, computed on request
-  DevBuf<double> ytmp;     // intermediate of precond (FP64 path)
-  DevBuf<float> ytmp32;    // intermediate of precond (FP32 path)
+  DevBuf<double> ytmp;     // intermediate of PCG's preconditioner (FP64 path)
+  DevBuf<float> ytmp32;    // the same (FP32 path)
   DevBuf<double> acc64;    // external partial sums of split stages
   DevBuf<float> acc32;
   DevBuf<double> acck64;   // the same for up to 32 right-hand sides (n x 32)
   DevBuf<float> acck32;
-  std::vector<BlkWork> work;  // of the block plan; the last is in use
+  std::vector<SolveWork> work;  // of trsv and precond; the last is in use
 };
 
 // Block plan of both directions.  Left out: G's rows are too dense for it, its

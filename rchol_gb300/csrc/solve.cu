@@ -566,8 +566,8 @@ void build_plan(rchol_factor_s &F, cudaStream_t s) {
   F.plan = P;
 }
 
-// Grows the plan's temporaries.  Growing frees buffers that captured PCG
-// graphs point to, so every cached graph of this factor is dropped with them
+// Grows PCG's intermediate vector.  Growing frees a buffer that captured PCG
+// graphs point to, so every cached graph of this factor is dropped with it
 // (a replay would otherwise read and write freed memory).  Callers hold P.lock.
 static void ensure_scratch(SolvePlan &P, bool fp32, int64_t count) {
   bool grew = false;
@@ -607,8 +607,8 @@ static void *ensure_acc(SolvePlan &P, bool fp32, int64_t n) {
   return P.acc64.p;
 }
 
-// What k right-hand sides need on the record streams.
-static void ensure_streams(const rchol_factor_s &F, int k, cudaStream_t s) {
+// What PCG needs for k right-hand sides.
+static void ensure_pcg(const rchol_factor_s &F, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   ensure_scratch(P, fp32, F.n * k);
@@ -616,30 +616,36 @@ static void ensure_streams(const rchol_factor_s &F, int k, cudaStream_t s) {
   else build_streams_k(F, P, s);
 }
 
-// What k right-hand sides need on the block plan.  Columns come in a power of
-// two.  A workspace that is grown out of stays until the factor goes, because
-// a caller's graph of a solve with fewer columns holds its addresses (all of
-// them together are smaller than the last).
-static void ensure_blocks(const rchol_factor_s &F, int k, cudaStream_t s) {
+// What trsv and precond need for k right-hand sides on the block plan or the
+// record streams: accumulator and workspace.  Columns come in a power of two.
+// A workspace that is grown out of stays until the factor goes, because a
+// caller's graph of a solve with fewer columns holds its addresses (all of
+// them together are smaller than the last); PCG does not share them.
+static const SolveWork &ensure_work(const rchol_factor_s &F, bool blocks, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   const size_t n = (size_t)F.n;
-  int cols = 1;
-  while (cols < std::min(k, kBlkCols)) cols *= 2;
   if (k == 1) {
     ensure_acc(P, fp32, F.n);
-  } else {
+  } else if (blocks) {
     build_blocks_k(F, P, std::min(k, kBlkCols), s);
     if (fp32 && P.acck32.n < n * kBlkCols) P.acck32.alloc(n * kBlkCols);
     if (!fp32 && P.acck64.n < n * kBlkCols) P.acck64.alloc(n * kBlkCols);
+  } else {
+    build_streams_k(F, P, s);
   }
-  if (!P.work.empty() && P.work.back().cols >= cols) return;
-  BlkWork w;
-  w.cols = cols;
-  if (fp32) w.y32.alloc(n * cols);
-  else w.y64.alloc(n * cols);
-  if (cols > 1) w.a.alloc(n * cols), w.b.alloc(n * cols);
-  P.work.push_back(std::move(w));
+  const int need = blocks ? std::min(k, kBlkCols) : k;
+  int cols = 1;
+  while (cols < need) cols *= 2;
+  if (P.work.empty() || P.work.back().cols < cols) {
+    SolveWork w;
+    w.cols = cols;
+    if (fp32) w.y32.alloc(n * cols);
+    else w.y64.alloc(n * cols);
+    if (blocks && k > 1) w.a.alloc(n * cols), w.b.alloc(n * cols);
+    P.work.push_back(std::move(w));
+  }
+  return P.work.back();
 }
 
 // Columns j0 .. j0 + g of an n x k row-major array, one after another
@@ -673,12 +679,11 @@ static void move_columns(int64_t n, int k, int j0, int g, const double *in, doub
 
 // k right-hand sides (n x k row-major) on the block plan, up to kBlkCols
 // columns at a time: the solve of direction `dir` (0, 1) or the preconditioner (2).
-static void blocks_k(const rchol_factor_s &F, const SolvePlan &P, int dir, const double *in, double *out, int k,
-                     cudaStream_t s) {
+static void blocks_k(const rchol_factor_s &F, const SolvePlan &P, const SolveWork &w, int dir, const double *in,
+                     double *out, int k, cudaStream_t s) {
   const int64_t n = F.n;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   void *acc = fp32 ? (void *)P.acck32.p : (void *)P.acck64.p;
-  const BlkWork &w = P.work.back();
   double *a = w.a.p, *b = w.b.p;
   for (int j0 = 0; j0 < k; j0 += kBlkCols) {
     const int g = std::min(kBlkCols, k - j0);
@@ -696,46 +701,41 @@ static void blocks_k(const rchol_factor_s &F, const SolvePlan &P, int dir, const
   }
 }
 
-// The preconditioner by the record streams, with the plan's buffers already
-// sized (inside PCG).
-static void precond_streams(const rchol_factor_s &F, const double *r, double *z, int k, cudaStream_t s) {
+// The preconditioner by the record streams with the intermediate vector(s) in
+// y64 or y32, everything sized already.
+static void precond_streams(const rchol_factor_s &F, const double *r, double *z, double *y64, float *y32, int k,
+                            cudaStream_t s) {
   SolvePlan &P = *F.plan;
   const bool fp32 = F.precision == RCHOL_PREC_FP32;
   if (k == 1) {
-    precond_one(F, P, false, r, z, P.ytmp.p, P.ytmp32.p, ensure_acc(P, fp32, F.n), s);
+    precond_one(F, P, false, r, z, y64, y32, ensure_acc(P, fp32, F.n), s);
   } else if (fp32) {
-    stream_trsv_k(F, P, false, r, nullptr, nullptr, P.ytmp32.p, k, s);
-    stream_trsv_k(F, P, true, nullptr, P.ytmp32.p, z, nullptr, k, s);
+    stream_trsv_k(F, P, false, r, nullptr, nullptr, y32, k, s);
+    stream_trsv_k(F, P, true, nullptr, y32, z, nullptr, k, s);
   } else {
-    stream_trsv_k(F, P, false, r, nullptr, P.ytmp.p, nullptr, k, s);
-    stream_trsv_k(F, P, true, P.ytmp.p, nullptr, z, nullptr, k, s);
+    stream_trsv_k(F, P, false, r, nullptr, y64, nullptr, k, s);
+    stream_trsv_k(F, P, true, y64, nullptr, z, nullptr, k, s);
   }
 }
 
 void trsv(const rchol_factor_s &F, bool upper, const double *in, double *out, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
-  const bool fp32 = F.precision == RCHOL_PREC_FP32;
   const bool blocks = k == 1 ? P.blocked1 : P.blocked;
-  if (blocks) ensure_blocks(F, k, s);
-  else ensure_streams(F, k, s);
-  if (k == 1) trsv_one(F, P, blocks, upper, in, nullptr, out, nullptr, ensure_acc(P, fp32, F.n), s);
-  else if (blocks) blocks_k(F, P, upper, in, out, k, s);
+  const SolveWork &w = ensure_work(F, blocks, k, s);
+  if (k == 1) trsv_one(F, P, blocks, upper, in, nullptr, out, nullptr, ensure_acc(P, F.precision == RCHOL_PREC_FP32, F.n), s);
+  else if (blocks) blocks_k(F, P, w, upper, in, out, k, s);
   else stream_trsv_k(F, P, upper, in, nullptr, out, nullptr, k, s);
 }
 
 void precond(const rchol_factor_s &F, const double *r, double *z, int k, cudaStream_t s) {
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
-  if (!(k == 1 ? P.blocked1 : P.blocked)) {
-    ensure_streams(F, k, s);
-    precond_streams(F, r, z, k, s);
-    return;
-  }
-  ensure_blocks(F, k, s);
-  const BlkWork &w = P.work.back();
-  if (k == 1) precond_one(F, P, true, r, z, w.y64.p, w.y32.p, ensure_acc(P, F.precision == RCHOL_PREC_FP32, F.n), s);
-  else blocks_k(F, P, 2, r, z, k, s);
+  const bool blocks = k == 1 ? P.blocked1 : P.blocked;
+  const SolveWork &w = ensure_work(F, blocks, k, s);
+  if (!blocks) precond_streams(F, r, z, w.y64.p, w.y32.p, k, s);
+  else if (k == 1) precond_one(F, P, true, r, z, w.y64.p, w.y32.p, ensure_acc(P, F.precision == RCHOL_PREC_FP32, F.n), s);
+  else blocks_k(F, P, w, 2, r, z, k, s);
 }
 
 // ---- preconditioner apply without allocation --------------------------------------------
@@ -922,7 +922,7 @@ static void pcg_iteration(const rchol_matrix_s &A, const rchol_factor_s &F, PcgW
   const int k = w.k;
   const int64_t n = A.n, nk = n * k;
   const unsigned eb = (unsigned)((nk + 255) / 256);
-  precond_streams(F, w.r.p, w.z.p, k, s);
+  precond_streams(F, w.r.p, w.z.p, F.plan->ytmp.p, F.plan->ytmp32.p, k, s);
   reduce_kernel<RED_DOT><<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, st, w.r.p, w.z.p, nullptr, nullptr, nullptr);
   finalize_kernel<<<k, RED_THREADS, 0, s>>>(st, FIN_BETA, 0, nullptr);
   pupdate_kernel<<<eb, 256, 0, s>>>(nk, st, w.p.p, w.z.p);
@@ -943,7 +943,7 @@ static void pcg_impl(const rchol_matrix_s &A, const rchol_factor_s &F, const dou
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
   const int64_t n = A.n, nk = n * k;
-  ensure_streams(F, k, s);
+  ensure_pcg(F, k, s);
   PcgWork &w = pcg_workspace(A, F, k);
   PcgState st = pcg_state(w);
   cudaStream_t ws = w.stream;
@@ -1355,7 +1355,7 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
   SolvePlan &P = *F.plan;
   std::lock_guard<std::mutex> guard(P.lock);
   const int64_t n = A.n;
-  ensure_streams(F, 1, s);
+  ensure_pcg(F, 1, s);
   SegWork &w = seg_workspace(A, F, nseg, seg);
   SegState st = seg_state(w);
   const unsigned S = (unsigned)nseg;
@@ -1373,7 +1373,7 @@ static void pcg_batch_impl(const rchol_matrix_s &A, const rchol_factor_s &F, int
     cudaGraph_t g = nullptr;
     RCHOL_CUDA(cudaStreamBeginCapture(ws, cudaStreamCaptureModeThreadLocal));
     try {
-      precond_streams(F, w.r.p, w.z.p, 1, ws);
+      precond_streams(F, w.r.p, w.z.p, P.ytmp.p, P.ytmp32.p, 1, ws);
       if (w.one_block) {
         seg_beta_one_kernel<<<S, SEG_THREADS, 0, ws>>>(st, w.r.p, w.z.p, w.p.p);
         spmv(A, w.p.p, w.q.p, 1, ws);

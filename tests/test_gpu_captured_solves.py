@@ -10,16 +10,19 @@ from rchol_gb300 import _lib, generators
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("streams", [False, True], ids=["blocks", "streams"])
 @pytest.mark.parametrize("k", [1, 2, 3])
 @pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
-def test_replay_after_wider_calls(cuda, R, precision, k):
+def test_replay_after_wider_calls(cuda, R, monkeypatch, precision, k, streams):
     import torch
 
+    if streams:
+        monkeypatch.setenv("RCHOL_TRSV_FORMAT", "1")
     A = generators.laplace_3d(18)
     tree = R.Tree.build(A.indptr, A.indices, 16)
     Ad = R.Matrix.create(A.indptr, A.indices, A.data, tree)
     F = R.Factor.compute(Ad, tree, seed=5, precision=precision)
-    assert F.blocked()
+    assert F.blocked() != streams
     lib, n = _lib.lib(), A.shape[0]
     rng = np.random.default_rng(3)
 
